@@ -64,6 +64,11 @@ GROUPS = {
     "kuramoto": [("atsit5", "plain", "kuramoto", 12, "fp64"),
                  ("atsit5", "persistent", "kuramoto", 12, "fp64")],
     "kuramoto_staged": [("atsit5", "staged", "kuramoto", 12, "fp64")],
+    # the same with the stages' linear combinations on the integer pipe, for ensembles that fill the GPU
+    # (use_integer_pipe in ode_capi.cu)
+    "lorenz_ic": [("atsit5", "plain", "lorenz", 3, "fp64"),
+                  ("atsit5", "persistent", "lorenz", 3, "fp64")],
+    "lorenz_staged_ic": [("atsit5", "staged", "lorenz", 3, "fp64")],
 }
 
 
@@ -72,12 +77,17 @@ GROUPS = {
 # shape the autotuner picks on the benchmark workloads (a ring that holds a
 # round plus a step's worth of new jobs, at no cost in occupancy); Kuramoto-12's
 # 804-byte jobs take one-warp blocks with a ring of exactly one round (32 jobs),
-# eight warps per SM.
-SHAPES = {"lorenz_staged": (64, 24576), "vdp_staged": (64, 24576), "kuramoto_staged": (32, 26112)}
+# eight warps per SM.  The integer-pipe kernel's warps also hold their stages in
+# shared memory, and it gains from every warp there is room for: the smallest
+# rings (36 jobs) in two-warp blocks give 16 warps per SM (1M learned Lorenz
+# solve: 104.8 ms with 8 warps per SM, 92.5 with 10, 84.6 with 12, 80.5 with 14,
+# 77.1 with 16).
+SHAPES = {"lorenz_staged": (64, 24576), "vdp_staged": (64, 24576), "kuramoto_staged": (32, 26112),
+          "lorenz_staged_ic": (64, 8704)}
 
 
-def kname(alg, kind, rhs, dim, prec):
-    return "gbode_%s_%s_%s%d_%s" % (alg, kind, rhs, dim, prec)
+def kname(alg, kind, rhs, dim, prec, ic=False):
+    return "gbode_%s_%s_%s%d_%s%s" % (alg, kind, rhs, dim, prec, "_ic" if ic else "")
 
 
 def write_if_changed(path, text):
@@ -95,6 +105,7 @@ def gen_sources():
                        ("tableaus.h", "kSrc_tableaus_h"), ("sde_solver.cuh", "kSrc_sde_solver_cuh"),
                        ("log_table.h", "kSrc_log_table_h"), ("exp_table.h", "kSrc_exp_table_h"),
                        ("ds_table.h", "kSrc_ds_table_h"), ("bitops.h", "kSrc_bitops_h"),
+                       ("intchain.h", "kSrc_intchain_h"), ("introws.h", "kSrc_introws_h"),
                        ("crpow.h", "kSrc_crpow_h"), ("crpow_table.h", "kSrc_crpow_table_h")):
         text = open(os.path.join(HERE, fname)).read()
         assert ")GBSRC\"" not in text
@@ -104,24 +115,26 @@ def gen_sources():
     decl, entries, tus = [], [], []
     for g, items in GROUPS.items():
         block, ring = SHAPES.get(g, (128, 12288))
+        ic = g.endswith("_ic")
         lines = ["/* generated by build.py: ahead-of-time kernels, group %s */\n" % g,
                  "#define GBODE_BLOCK %d\n#define GBODE_STAGE_BYTES %d\n" % (block, ring),
                  "#define GBODE_CTRL_DS 1 /* the default error norm and controller (ODE_CTRL_DS) */\n",
+                 "#define GBODE_IC 1\n" if ic else "",
                  '#include "ode_solver.cuh"\n']
         for i, (alg, kind, rhs, dim, prec) in enumerate(items):
             t = "RHS_%s_%d" % (g, i)
             lines.append("typedef %s %s;\n" % (rhs_type(rhs, dim, prec), t))
-            lines.append("GBODE_ENTRY(%s, %s, %s, %s, %s)\n" % (kname(alg, kind, rhs, dim, prec), kind,
+            lines.append("GBODE_ENTRY(%s, %s, %s, %s, %s)\n" % (kname(alg, kind, rhs, dim, prec, ic), kind,
                                                                METHOD[alg], PREC[prec][1], t))
-            decl.append('extern "C" __global__ void %s(gbode::KParams);\n' % kname(alg, kind, rhs, dim, prec))
-            entries.append('  {%d, "%s", %d, %d, %d, (const void*)%s, %d, %d},\n' % (
-                ALG[alg], kind, RHS[rhs], dim, PREC[prec][0], kname(alg, kind, rhs, dim, prec), block, ring))
+            decl.append('extern "C" __global__ void %s(gbode::KParams);\n' % kname(alg, kind, rhs, dim, prec, ic))
+            entries.append('  {%d, "%s", %d, %d, %d, (const void*)%s, %d, %d, %d},\n' % (
+                ALG[alg], kind, RHS[rhs], dim, PREC[prec][0], kname(alg, kind, rhs, dim, prec, ic), block, ring, int(ic)))
         path = os.path.join(BUILD, "kern_%s.cu" % g)
         write_if_changed(path, "".join(lines))
         tus.append(path)
     reg = ["/* generated by build.py: kernels compiled ahead of time */\n",
            "struct AotEntry { int alg; const char* kind; int rhs; int dim; int precision; const void* fn; int block; "
-           "int stage; };\n"]
+           "int stage; int ic; };\n"]
     reg += decl
     reg.append("static const AotEntry kAotEntries[] = {\n")
     reg += entries
@@ -156,7 +169,8 @@ def build(verbose=False, jobs=None):
     os.makedirs(LIB, exist_ok=True)
     headers = [os.path.join(HERE, f) for f in ("ode_solver.cuh", "ode_kparams.h", "tableaus.h", "ode_host.h",
                                                "jlrange.h", "sde_solver.cuh", "log_table.h", "exp_table.h",
-                                               "ds_table.h", "bitops.h", "crpow.h", "crpow_table.h")] + [
+                                               "ds_table.h", "bitops.h", "intchain.h", "introws.h", "crpow.h",
+                                               "crpow_table.h")] + [
         os.path.join(PKG, "..", "include", "gb300ode.h")]
     host_tus = [os.path.join(HERE, f) for f in ("ode_capi.cu", "learn.cu", "noalloc.cu", "sde_capi.cu")]
     gen = [os.path.join(BUILD, "aot_registry.inc"), os.path.join(BUILD, "embedded_src.inc")]

@@ -330,16 +330,57 @@ int stage_unit_bytes(const ode_solve_args* a) {
   return rec ? rec : stage_job_bytes(a);
 }
 
+/* Bytes of shared memory a warp of the integer-pipe kernels keeps its stages
+ * in: the host-side copy of Stages<...>::BYTES in ode_solver.cuh. */
+int stage_slice_bytes(const ode_solve_args* a) { return 7 * a->dim * 32 * 8; }
+
+/* A ring of 36 units, in steps of 512 bytes: a round of 32 and a few more. */
+int small_ring_bytes(const ode_solve_args* a) { return (36 * stage_unit_bytes(a) + 511) / 512 * 512; }
+
+/* Whether this solve runs the kernel that keeps the stages in shared memory
+ * and forms their linear combinations on the integer pipe (GBODE_IC,
+ * intchain.h): adaptive Tsit5 in FP64, in the default rounding.
+ *
+ * It pays once the FP64 pipe is shared.  A lone warp waits as long for a
+ * linear combination of integers as for one of fused multiply-adds; with more
+ * than two warps on an SM sub-partition the pipe bounds the solve and the
+ * integer pipe relieves it.  Time of the register kernel over this one's:
+ *   n                      25,000  35,000  45,000  80,000  250,000
+ *   Lorenz, 50 saveat        0.91    1.12    1.13    1.25    1.31
+ *   Lorenz, plain, saveat    0.99    1.19    1.32    1.37    1.41
+ *   Lotka-Volterra, saveat   0.95    0.94    1.12    1.04    1.08
+ *   linear, dim 4, saveat    1.05    1.05    1.08    1.06    1.23
+ *   linear, dim 6            1.03    1.04    1.04    1.05    1.15
+ * (two warps on each of the 608 sub-partitions are 38,912 trajectories).  The
+ * size limit keeps at least 12 warps an SM: with fewer the integer pipe's
+ * latency shows (the Lorenz solve above at 8: no gain). */
+bool use_integer_pipe(const ode_handle* h, const ode_solve_args* a, int sched) {
+  if (a->alg != ODE_ALG_ATSIT5 || a->precision != ODE_FP64 || a->controller == ODE_CTRL_REF) return false;
+  const bool staged = !std::strcmp(entry_kind(a->alg, sched, a->nsave), "staged");
+  if (stage_slice_bytes(a) + (staged ? small_ring_bytes(a) : 0) > 19456) return false;
+  if (h->tune_int >= 0) return h->tune_int != 0;
+  return a->n > (int64_t)h->nsm * 4 * 64;
+}
+
 /* Launch shape of an untuned run-time compiled kernel: 128 threads and 12 KB
  * staging rings, unless those rings cannot hold a round of 32 (a staged kernel
  * with large records): then one-warp blocks with the smallest ring that can,
  * up to 48 KB (measured on AVern9, restricted three-body problem, 65,536
  * trajectories, 100 save points: 161.7 ms unstaged, 116.4 ms staged in
- * one-warp blocks with 29 KB rings, 121.3 with 36 KB, 128.8 with 48 KB). */
-void default_shape(const ode_solve_args* a, int sched, int* block, int* stage) {
+ * one-warp blocks with 29 KB rings, 121.3 with 36 KB, 128.8 with 48 KB).
+ * The integer-pipe kernels, whose warps also hold their stages in shared
+ * memory, take two-warp blocks with the smallest ring. */
+void default_shape(const ode_handle* h, const ode_solve_args* a, int sched, int* block, int* stage) {
   *block = 128;
   *stage = 12288;
-  if (std::strcmp(entry_kind(a->alg, sched, a->nsave), "staged") != 0) return;
+  const bool staged = !std::strcmp(entry_kind(a->alg, sched, a->nsave), "staged");
+  if (use_integer_pipe(h, a, sched)) {
+    if (staged) *stage = small_ring_bytes(a);
+    while (*block > 32 && *block / 32 * (stage_slice_bytes(a) + (staged ? *stage : 0)) > (staged ? 40960 : 49152))
+      *block /= 2;
+    return;
+  }
+  if (!staged) return;
   const int unit = stage_unit_bytes(a);
   if (((12288 / unit) & ~7) >= 32) return;
   const int fit = (32 * unit + 511) / 512 * 512;
@@ -372,9 +413,9 @@ const char* ctrl_suffix(int v) {
 
 std::string kernel_key(ode_handle* h, const ode_solve_args* a, int sched) {
   char b[160];
-  snprintf(b, sizeof b, "%s|%s|%d|%d|%s|%d%s%s", alg_name(a->alg), kernel_kind(h, a, sched), a->rhs, a->dim,
+  snprintf(b, sizeof b, "%s|%s|%d|%d|%s|%d%s%s%s", alg_name(a->alg), kernel_kind(h, a, sched), a->rhs, a->dim,
            prec_name(a->precision), a->output >= ODE_OUTPUT_USER ? a->output : 0, h->bounds_check ? "|chk" : "",
-           ctrl_suffix(ctrl_variant(a)));
+           ctrl_suffix(ctrl_variant(a)), use_integer_pipe(h, a, sched) ? "|ic" : "");
   return b;
 }
 
@@ -382,6 +423,7 @@ std::string kernel_key(ode_handle* h, const ode_solve_args* a, int sched) {
  * dim, schedule kind). */
 std::string jit_source(ode_handle* h, const ode_solve_args* a, int sched) {
   std::string src;
+  if (use_integer_pipe(h, a, sched)) src += "#define GBODE_IC 1\n";
   if (ctrl_variant(a) == ODE_CTRL_FP64) src += "#define GBODE_CTRL64 1\n";
   if (ctrl_variant(a) == ODE_CTRL_DS) src += "#define GBODE_CTRL_DS 1\n";
   if (ctrl_variant(a) == ODE_CTRL_REF) src += "#define GBODE_REF 1\n";
@@ -429,10 +471,11 @@ int nvrtc_cubin(const std::string& src, const std::vector<std::string>& extra_op
   }
   nvrtcProgram prog;
   const char* hdrs[] = {kSrc_ode_solver_cuh, kSrc_ode_kparams_h, kSrc_tableaus_h, kSrc_sde_solver_cuh, kSrc_log_table_h,
-                        kSrc_exp_table_h, kSrc_ds_table_h, kSrc_bitops_h, kSrc_crpow_h, kSrc_crpow_table_h};
+                        kSrc_exp_table_h, kSrc_ds_table_h, kSrc_bitops_h, kSrc_crpow_h, kSrc_crpow_table_h,
+                        kSrc_intchain_h, kSrc_introws_h};
   const char* names[] = {"ode_solver.cuh", "ode_kparams.h", "tableaus.h", "sde_solver.cuh", "log_table.h",
-                         "exp_table.h", "ds_table.h", "bitops.h", "crpow.h", "crpow_table.h"};
-  nvrtcResult r = g_nvrtc.create(&prog, src.c_str(), "gbode_jit.cu", 10, hdrs, names);
+                         "exp_table.h", "ds_table.h", "bitops.h", "crpow.h", "crpow_table.h", "intchain.h", "introws.h"};
+  nvrtcResult r = g_nvrtc.create(&prog, src.c_str(), "gbode_jit.cu", 12, hdrs, names);
   if (r != NVRTC_SUCCESS) {
     *err = std::string("nvrtcCreateProgram: ") + g_nvrtc.errstr(r);
     return ODE_ENVRTC;
@@ -475,7 +518,7 @@ int compile_jit(ode_handle* h, const ode_solve_args* a, int sched, CUfunction* f
   std::vector<char> cubin;
   std::string err;
   int block = 128, stage = 12288;
-  default_shape(a, sched, &block, &stage);
+  default_shape(h, a, sched, &block, &stage);
   std::vector<std::string> opts = {"-DGBODE_BLOCK=" + std::to_string(block),
                                    "-DGBODE_STAGE_BYTES=" + std::to_string(stage)};
   if (h->bounds_check) opts.push_back("-DGBODE_BOUNDS_CHECK");
@@ -516,11 +559,12 @@ int get_kernel(ode_handle* h, const ode_solve_args* a, int sched, CUfunction* fn
     return ODE_OK;
   }
   const char* kind = kernel_kind(h, a, sched);
+  const bool ic = use_integer_pipe(h, a, sched);
   for (const AotEntry& e : kAotEntries) {
     if (!h->bounds_check && ctrl_variant(a) == ODE_CTRL_DS && a->output < ODE_OUTPUT_USER && e.alg == a->alg &&
         e.rhs == a->rhs &&
         e.dim == a->dim &&
-        e.precision == a->precision && std::strcmp(e.kind, kind) == 0) {
+        e.precision == a->precision && std::strcmp(e.kind, kind) == 0 && (e.ic != 0) == ic) {
       cudaFunction_t f;
       cudaError_t ce = cudaGetFuncBySymbol(&f, e.fn);
       if (ce != cudaSuccess) return cuda_fail(h, ce, "cudaGetFuncBySymbol");
@@ -629,13 +673,14 @@ static std::string gpu_tag(ode_handle* h) {
   return name + "/" + std::to_string(prop.multiProcessorCount);
 }
 
-/* kernel keys are alg|kind|rhs|dim|prec|output[|chk][|c64, |c32 or |ref]; only built-in ids travel,
+/* kernel keys are alg|kind|rhs|dim|prec|output[|chk][|c64, |c32 or |ref][|ic]; only built-in ids travel,
  * and no bounds-check build */
 static bool portable_key(const std::string& key) {
   std::vector<std::string> f;
   size_t a = 0;
   for (size_t b; (b = key.find('|', a)) != std::string::npos; a = b + 1) f.push_back(key.substr(a, b - a));
   f.push_back(key.substr(a));
+  if (f.size() > 6 && f.back() == "ic") f.pop_back();
   const bool has_ctrl = f.size() == 7 && (f[6] == "c64" || f[6] == "c32" || f[6] == "ref");
   return (f.size() == 6 || has_ctrl) && std::atoi(f[2].c_str()) < ODE_RHS_USER &&
          std::atoi(f[5].c_str()) < ODE_OUTPUT_USER;
@@ -1579,6 +1624,13 @@ int ode_autotune(ode_handle* h, const ode_solve_args* a, int64_t sample, ode_tun
   std::memset(&to, 0, sizeof to);
   to.us = dus;
   to.u_final = duf;
+  /* the whole ensemble's kernel is tuned, whatever the sample's size would choose */
+  struct TuneInt {
+    ode_handle* h;
+    ~TuneInt() { h->tune_int = -1; }
+  } tune_int{h};
+  h->tune_int = use_integer_pipe(h, a, ta.schedule);
+  const bool ic = use_integer_pipe(h, &ta, ta.schedule);
   const std::string key = kernel_key(h, &ta, ta.schedule);
   /* the baseline is the kernel an untuned handle would run */
   h->tuned.erase(key);
@@ -1617,7 +1669,7 @@ int ode_autotune(ode_handle* h, const ode_solve_args* a, int64_t sample, ode_tun
   for (int block : {128, 64, 32}) {
     std::vector<int> rings;
     if (staged) {
-      if (fit > 12288 && fit / 32 * block <= 49152) rings.push_back(fit);
+      if ((ic || fit > 12288) && fit / 32 * block <= 49152) rings.push_back(fit);
       for (int ring : {12288, 16384, 24576, 36864, 49152})
         if (ring / 32 * block <= 49152 && (ring / job & ~7) >= 32) rings.push_back(ring);
     }

@@ -55,6 +55,7 @@
 #pragma once
 #include "ode_kparams.h"
 #include "bitops.h"
+#include "introws.h"
 #ifdef GBODE_REF
 #include "crpow.h"
 #endif
@@ -816,7 +817,7 @@ template <class PR, int D, class F>
 struct MTsit5 {
   typedef typename PR::R R;
   typedef typename PR::T T;
-  enum { NK = 7, FSAL = 1, DTMIN_1F7 = 0, DENSE_F = 0 };  /* DENSE_F: dense output evaluates f */
+  enum { NK = 7, FSAL = 1, DTMIN_1F7 = 0, DENSE_F = 0, NX = 0, IC = 1 };  /* DENSE_F: dense output evaluates f */
 
   __device__ static __forceinline__ void attempt(const F& f, const R (&uh)[D], const R (&uc)[D], T t, T dt,
                                                  R (&k)[NK][D], R (&nh)[D], R (&nc)[D], R (&e)[D], bool want_err) {
@@ -884,7 +885,7 @@ template <class PR, int D, class F>
 struct MVern7 {
   typedef typename PR::R R;
   typedef typename PR::T T;
-  enum { NK = 10, FSAL = 0, DTMIN_1F7 = 0, DENSE_F = 1 };
+  enum { NK = 10, FSAL = 0, DTMIN_1F7 = 0, DENSE_F = 1, IC = 0 };
 
   __device__ static __forceinline__ void attempt(const F& f, const R (&uh)[D], const R (&uc)[D], T t, T dt,
                                                  R (&k)[NK][D], R (&nh)[D], R (&nc)[D], R (&e)[D], bool want_err) {
@@ -1006,7 +1007,7 @@ template <class PR, int D, class F, bool ADAPTIVE>
 struct MVern9Impl {
   typedef typename PR::R R;
   typedef typename PR::T T;
-  enum { NK = 16, FSAL = 0, DTMIN_1F7 = 1, DENSE_F = 1 };
+  enum { NK = 16, FSAL = 0, DTMIN_1F7 = 1, DENSE_F = 1, IC = 0 };
 
   __device__ static __forceinline__ void attempt(const F& f, const R (&uh)[D], const R (&uc)[D], T t, T dt,
                                                  R (&k)[NK][D], R (&nh)[D], R (&nc)[D], R (&e)[D], bool want_err) {
@@ -1243,13 +1244,192 @@ struct MEuler {
   }
 };
 
+/* Launch shape: threads per block and the bytes of each warp's staging ring.
+ * Both can be set at compile time (the autotuner compiles variants); the
+ * defaults give 4 warps x 12 KB = 48 KB of static shared memory per block. */
+#ifndef GBODE_BLOCK
+#define GBODE_BLOCK 128
+#endif
+#ifndef GBODE_STAGE_BYTES
+#define GBODE_STAGE_BYTES 12288
+#endif
+constexpr int kStageBytesPerWarp = GBODE_STAGE_BYTES;
+constexpr int kWarpsPerBlock = GBODE_BLOCK / 32;
+
+
+/* ------------------------------------------------------------------ stages on the integer pipe */
+/* Stage values in memory: value d of stage q at p[(q * D + d) * STRIDE]. */
+template <class R, int STRIDE>
+struct StageRow {
+  R* p;
+  __device__ __forceinline__ R& operator[](int d) const { return p[d * STRIDE]; }
+};
+template <class R, int D, int STRIDE>
+struct StageRows {
+  R* p;
+  /* whether a linear combination of the last attempt was not decided on the
+   * integer pipe; attempts left that do without it */
+  bool missed;
+  int rest;
+  __device__ __forceinline__ StageRow<R, STRIDE> operator[](int q) const { return StageRow<R, STRIDE>{p + q * D * STRIDE}; }
+};
+
+static_assert(tsit5_btilde7 == tsit5_btilde1 + 6, "the error weights are consecutive");
+
+/* Tsit5's attempt with the stages in shared memory and their linear
+ * combinations on the integer pipe (intchain.h): the same values as
+ * MTsit5::attempt.  The FP64 pipe bounds the solve; of an attempt's 162 FP64
+ * instructions on Lorenz this leaves 99: the right-hand sides, the state
+ * updates u + h s (whose two terms can be 2^40 apart) and the error estimate
+ * (whose sum cancels 20 bits and more: undecided in 8 rows of 10).
+ *
+ * The loops over rows and terms stay rolled, one right-hand side in the code:
+ * unrolled, the chains were 30 KB more code and the warps, at different points
+ * of it, waited for instructions (98 ms for the 1M learned Lorenz solve
+ * against 77 ms rolled, 108 ms with multiply-adds in registers).  Rolled
+ * loops need indexable stages, and shared memory holds them (7 x D doubles a
+ * lane), which also frees the registers for 16 warps an SM instead of 8. */
+template <class M, class PR, int D, class F>
+struct MInt : M {
+  typedef typename PR::R R;
+  typedef typename PR::T T;
+
+  /* s = sum_j c_j k_j of a row, whose term j multiplies stage j, by fused
+   * multiply-adds as lc() does it */
+  template <int STRIDE>
+  __device__ static __forceinline__ void row_fma(const IcRow& row, const R* kb, R (&s)[D]) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) s[d] = c_ic_t5.coef[row.first] * kb[d * STRIDE];
+#pragma unroll 1
+    for (int j = 1; j < row.n; ++j) {
+      const R c = c_ic_t5.coef[row.first + j];
+      const R* kp = kb + j * D * STRIDE;
+#pragma unroll
+      for (int d = 0; d < D; ++d) s[d] = fmaR(c, kp[d * STRIDE], s[d]);
+    }
+  }
+  /* the same on the integer pipe; false if a component's sum was not decided there */
+  template <int STRIDE>
+  __device__ static __forceinline__ bool row_int(const IcRow& row, const R* kb, const IcSpan (&E)[D], R (&s)[D]) {
+    IcSum S[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) S[d] = IcSum{0u, 0u, 0u, false};
+#pragma unroll 1
+    for (int j = 0; j < row.n; ++j) {
+      const IcTerm c = c_ic_t5.term[row.first + j];
+      const R* kp = kb + j * D * STRIDE;
+#pragma unroll
+      for (int d = 0; d < D; ++d) ic_add_product(S[d], ic_product(c, kp[d * STRIDE], E[d]));
+    }
+    bool ok = true;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      s[d] = ic_result(S[d], E[d], row.emax);
+      ok = ok && !S[d].bad && ic_in_window(E[d], row.shift);
+    }
+    return ok;
+  }
+  /* whichever applies; false if the integer pipe was tried and left the row undecided */
+  template <int STRIDE>
+  __device__ static __forceinline__ bool row_sum(const IcRow& row, const R* kb, const IcSpan (&E)[D], bool on_int,
+                                                 R (&s)[D]) {
+    bool done = false;
+    if (on_int) done = row_int<STRIDE>(row, kb, E, s);
+    if (!done) row_fma<STRIDE>(row, kb, s);
+    return done || !on_int;
+  }
+
+  template <int STRIDE>
+  __device__ static __forceinline__ void attempt(const F& f, const R (&uh)[D], const R (&uc)[D], T t, T dt,
+                                                 StageRows<R, D, STRIDE>& k, R (&nh)[D], R (&nc)[D], R (&e)[D],
+                                                 bool want_err) {
+    const R h = (R)dt;
+    /* A row with a zero stage is never decided on the integer pipe.  Where
+     * that keeps happening (a component at rest), the lane, and with it the
+     * lanes it runs with, does without it for the next attempts. */
+    const bool on_int = !__any_sync(__activemask(), k.rest > 0);
+    bool missed = false;
+    R tmp[D], du[D];
+    IcSpan E[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) E[d] = ic_span(k[0][d]);
+#pragma unroll 1
+    for (int r = 0; r < kRowsT5; ++r) {
+      const IcRow row = c_ic_t5.row[r];
+      if (r == 0) {
+        const R a = (R)(dt * c_ic_t5.coef[0]);
+#pragma unroll
+        for (int d = 0; d < D; ++d) tmp[d] = fmaR(a, k[0][d], uh[d]);
+      } else {
+        R s[D];
+        missed = !row_sum<STRIDE>(row, k.p, E, on_int, s) || missed;
+        axpy(tmp, uh, h, s);
+      }
+      f(tmp, stime(t, row.c, dt), du);
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        k.p[((r + 1) * D + d) * STRIDE] = du[d];
+        ic_widen(E[d], du[d]);
+      }
+    }
+    k.rest = missed && k.missed ? 31 : k.rest - (k.rest > 0);
+    k.missed = missed;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      nh[d] = tmp[d];
+      nc[d] = (R)0;
+      e[d] = c_tsit5_d[tsit5_btilde1] * k[0][d];
+    }
+#pragma unroll 1
+    for (int j = 1; j < M::NK; ++j) {
+      const R c = c_tsit5_d[tsit5_btilde1 + j];
+      const R* kp = k.p + j * D * STRIDE;
+#pragma unroll
+      for (int d = 0; d < D; ++d) e[d] = fmaR(c, kp[d * STRIDE], e[d]);
+    }
+    if (!ErrUnscaled<R>::value) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) e[d] = h * e[d];
+    }
+  }
+};
+
+/* Whether the adaptive kernels of this method and size keep the stages in
+ * shared memory and run their linear combinations on the integer pipe, and
+ * the types that follow from it.  RING: the staging ring's bytes per warp. */
+template <class M, class PR, int D, class F, int RING>
+struct Stages {
+  enum { BYTES = M::NK * D * 32 * 8 };
+#if defined(GBODE_IC) && !defined(GBODE_REF)
+  enum { SHARED = M::IC && sizeof(typename PR::R) == 8 && (GBODE_BLOCK / 32) * (BYTES + RING) <= 49152 };
+#else
+  enum { SHARED = 0 };
+#endif
+};
+template <bool SHARED, class M, class PR, int D, class F> struct StageTypes {
+  typedef M Method;
+  typedef typename PR::R KS[M::NK][D];
+  enum { SLICE = 1 };
+  __device__ static __forceinline__ void bind(KS&, typename PR::R*) {}
+};
+template <class M, class PR, int D, class F> struct StageTypes<true, M, PR, D, F> {
+  typedef MInt<M, PR, D, F> Method;
+  typedef StageRows<typename PR::R, D, 32> KS;
+  enum { SLICE = M::NK * D * 32 };
+  __device__ static __forceinline__ void bind(KS& k, typename PR::R* slice) {
+    k.p = slice + (threadIdx.x & 31);
+    k.missed = false;
+    k.rest = 0;
+  }
+};
+
 /* ------------------------------------------------------------------ per-lane trajectory state */
-template <class PR, int D, class F, int NK>
+template <class PR, int D, class F, int NK, class KS = typename PR::R[NK][D]>
 struct Lane {
   typedef typename PR::R R;
   typedef typename PR::T T;
   R uh[D], uc[D];
-  R k[NK][D];
+  KS k; /* stage values: registers, or a view of shared memory (StageRows) */
   F f;
   T t, dt;
   float qoldp;
@@ -1338,8 +1518,8 @@ __device__ __forceinline__ void store_step(const KParams& P, const L& l, long lo
 }
 
 /* Load trajectory idx: parameters, u0, t0, dt; first saveat point if it is t0. */
-template <class PR, int D, class F, int NK>
-__device__ __forceinline__ void lane_load(const KParams& P, long long idx, Lane<PR, D, F, NK>& l) {
+template <class PR, int D, class F, int NK, class KS>
+__device__ __forceinline__ void lane_load(const KParams& P, long long idx, Lane<PR, D, F, NK, KS>& l) {
   if (!GBODE_CHECK(P, idx >= 0 && idx < P.n, CHK_TRAJ)) idx = 0;
 #ifdef GBODE_BOUNDS_CHECK
   atomicAdd(&P.visited[idx], 1u);
@@ -1406,8 +1586,8 @@ __device__ __forceinline__ void flush_totals(const KParams& P, Totals t) {
   }
 }
 
-template <class PR, int D, class F, int NK>
-__device__ __forceinline__ void lane_finish(const KParams& P, Lane<PR, D, F, NK>& l, int ret, Totals& tot) {
+template <class PR, int D, class F, int NK, class KS>
+__device__ __forceinline__ void lane_finish(const KParams& P, Lane<PR, D, F, NK, KS>& l, int ret, Totals& tot) {
   const long long idx = l.idx;
   double v[D];
   state_value<PR, D>(l, v);
@@ -1451,8 +1631,8 @@ struct Accepted {
  * new state are left to the caller (the state before the step, the stage
  * values and the proposal nh/nc are still intact).  TRY_STOPPED: dt fell
  * below dtmin or the attempt cap was reached; the outputs are written. */
-template <class M, class PR, int D, class F, int NK>
-__device__ __forceinline__ int adaptive_try(const KParams& P, Lane<PR, D, F, NK>& l, Totals& tot,
+template <class M, class PR, int D, class F, int NK, class KS>
+__device__ __forceinline__ int adaptive_try(const KParams& P, Lane<PR, D, F, NK, KS>& l, Totals& tot,
                                             typename PR::R (&nh)[D], typename PR::R (&nc)[D],
                                             Accepted<typename PR::T>& acc_out) {
   typedef typename PR::R R;
@@ -1755,8 +1935,8 @@ __device__ __forceinline__ int adaptive_try(const KParams& P, Lane<PR, D, F, NK>
 }
 
 /* Replace the state by the accepted proposal (and the FSAL stage). */
-template <class M, class PR, int D, class F, int NK>
-__device__ __forceinline__ void adaptive_commit(Lane<PR, D, F, NK>& l, const typename PR::R (&nh)[D],
+template <class M, class PR, int D, class F, int NK, class KS>
+__device__ __forceinline__ void adaptive_commit(Lane<PR, D, F, NK, KS>& l, const typename PR::R (&nh)[D],
                                                 const typename PR::R (&nc)[D]) {
 #pragma unroll
   for (int d = 0; d < D; ++d) {
@@ -1771,8 +1951,8 @@ __device__ __forceinline__ void adaptive_commit(Lane<PR, D, F, NK>& l, const typ
 
 /* One attempt with the saveat points of an accepted step interpolated at once
  * by this lane.  Returns true when the trajectory has finished (outputs written). */
-template <class M, class PR, int D, class F, int NK>
-__device__ __forceinline__ bool adaptive_iter(const KParams& P, Lane<PR, D, F, NK>& l, Totals& tot) {
+template <class M, class PR, int D, class F, int NK, class KS>
+__device__ __forceinline__ bool adaptive_iter(const KParams& P, Lane<PR, D, F, NK, KS>& l, Totals& tot) {
   typedef typename PR::R R;
   typedef typename PR::T T;
   R nh[D], nc[D];
@@ -1798,11 +1978,16 @@ __device__ __forceinline__ bool adaptive_iter(const KParams& P, Lane<PR, D, F, N
 }
 
 /* Start trajectory idx; returns true if it is already finished (t0 >= tf). */
-template <class M, class PR, int D, class F, int NK>
-__device__ __forceinline__ bool adaptive_start(const KParams& P, long long idx, Lane<PR, D, F, NK>& l, Totals& tot) {
+template <class M, class PR, int D, class F, int NK, class KS>
+__device__ __forceinline__ bool adaptive_start(const KParams& P, long long idx, Lane<PR, D, F, NK, KS>& l, Totals& tot) {
   lane_load(P, idx, l);
   if (!(l.t < (typename PR::T)P.tf)) { lane_finish(P, l, RET_DEFAULT, tot); return true; }
-  if (M::FSAL) l.f(l.uh, l.t, l.k[0]);
+  if (M::FSAL) {
+    typename PR::R du[D];
+    l.f(l.uh, l.t, du);
+#pragma unroll
+    for (int d = 0; d < D; ++d) l.k[0][d] = du[d];
+  }
   return false;
 }
 
@@ -1810,11 +1995,15 @@ __device__ __forceinline__ bool adaptive_start(const KParams& P, long long idx, 
 template <class M, class PR, int D, class F>
 __device__ __forceinline__ void run_adaptive_plain(const KParams& P) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  typedef StageTypes<Stages<M, PR, D, F, 0>::SHARED, M, PR, D, F> ST;
+  typedef typename ST::Method MM;
+  __shared__ typename PR::R kmem[kWarpsPerBlock][ST::SLICE];
   Totals tot = {0, 0, 0};
   if (i < P.n) {
-    Lane<PR, D, F, M::NK> l;
-    if (!adaptive_start<M>(P, i, l, tot)) {
-      while (!adaptive_iter<M>(P, l, tot)) {
+    Lane<PR, D, F, M::NK, typename ST::KS> l;
+    ST::bind(l.k, kmem[threadIdx.x >> 5]);
+    if (!adaptive_start<MM>(P, i, l, tot)) {
+      while (!adaptive_iter<MM>(P, l, tot)) {
       }
     }
   }
@@ -1826,11 +2015,14 @@ __device__ __forceinline__ void run_adaptive_plain(const KParams& P) {
  * (one atomicAdd per warp for all lanes that need work) and the position is
  * mapped through P.order.  Every lane of a warp runs the loop until the whole
  * warp has no work left, so the warp-wide ballots stay convergent. */
-template <class M, class PR, int D, class F>
-__device__ __forceinline__ void run_adaptive_persistent(const KParams& P) {
+template <class M, class PR, int D, class F, int RING>
+__device__ __forceinline__ void run_adaptive_persistent(const KParams& P, typename PR::R* slice) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  Lane<PR, D, F, M::NK> l;
+  typedef StageTypes<Stages<M, PR, D, F, RING>::SHARED, M, PR, D, F> ST;
+  typedef typename ST::Method MM;
+  Lane<PR, D, F, M::NK, typename ST::KS> l;
+  ST::bind(l.k, slice);
   Totals tot = {0, 0, 0};
   bool active = false, exhausted = false;
   for (;;) {
@@ -1846,7 +2038,7 @@ __device__ __forceinline__ void run_adaptive_persistent(const KParams& P) {
         if (w < (unsigned long long)P.n) {
           long long idx = P.order ? (long long)P.order[w] : (long long)w;
           if (!GBODE_CHECK(P, idx >= 0 && idx < P.n, CHK_ORDER)) idx = 0;
-          active = !adaptive_start<M>(P, idx, l, tot);
+          active = !adaptive_start<MM>(P, idx, l, tot);
         } else {
           exhausted = true;
         }
@@ -1856,7 +2048,7 @@ __device__ __forceinline__ void run_adaptive_persistent(const KParams& P) {
       if (!__any_sync(FULL, !exhausted)) break;
       continue;
     }
-    if (active && adaptive_iter<M>(P, l, tot)) active = false;
+    if (active && adaptive_iter<MM>(P, l, tot)) active = false;
   }
   flush_totals(P, tot);
 }
@@ -1873,18 +2065,6 @@ __device__ __forceinline__ void run_adaptive_persistent(const KParams& P) {
  * jobs are waiting the whole warp interpolates 32 points at once, one per
  * lane.  Each point is computed by the same M::dense call on the same values,
  * so the results are bit-identical to the other drivers. */
-/* Launch shape: threads per block and the bytes of each warp's staging ring.
- * Both can be set at compile time (the autotuner compiles variants); the
- * defaults give 4 warps x 12 KB = 48 KB of static shared memory per block. */
-#ifndef GBODE_BLOCK
-#define GBODE_BLOCK 128
-#endif
-#ifndef GBODE_STAGE_BYTES
-#define GBODE_STAGE_BYTES 12288
-#endif
-constexpr int kStageBytesPerWarp = GBODE_STAGE_BYTES;
-constexpr int kWarpsPerBlock = GBODE_BLOCK / 32;
-
 template <class M, class PR, int D, class F>
 struct StageLayout {
   typedef typename PR::R R;
@@ -1915,7 +2095,7 @@ struct RingStages {
 };
 
 template <class M, class PR, int D, class F>
-__device__ __forceinline__ void run_adaptive_staged(const KParams& P) {
+__device__ __forceinline__ void run_adaptive_staged(const KParams& P, typename PR::R* slice) {
   typedef typename PR::R R;
   typedef typename PR::T T;
   typedef StageLayout<M, PR, D, F> SL;
@@ -1930,7 +2110,10 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P) {
   int* jv = (int*)(qb + 3 * CAP * sizeof(T) + 8 * CAP + SL::NREC * CAP * sizeof(R)); /* saveat index */
   int qhead = 0, qcount = 0; /* warp-uniform */
 
-  Lane<PR, D, F, NK> l;
+  typedef StageTypes<Stages<M, PR, D, F, kStageBytesPerWarp>::SHARED, M, PR, D, F> ST;
+  typedef typename ST::Method MM;
+  Lane<PR, D, F, NK, typename ST::KS> l;
+  ST::bind(l.k, slice);
   Totals tot = {0, 0, 0};
   bool active = false, exhausted = false;
 
@@ -1977,7 +2160,7 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P) {
         if (w < (unsigned long long)P.n) {
           long long idx = P.order ? (long long)P.order[w] : (long long)w;
           if (!GBODE_CHECK(P, idx >= 0 && idx < P.n, CHK_ORDER)) idx = 0;
-          active = !adaptive_start<M>(P, idx, l, tot);
+          active = !adaptive_start<MM>(P, idx, l, tot);
         } else {
           exhausted = true;
         }
@@ -1991,7 +2174,7 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P) {
     Accepted<T> st;
     int r = TRY_REJECTED, njobs = 0;
     if (active) {
-      r = adaptive_try<M>(P, l, tot, nh, nc, st);
+      r = adaptive_try<MM>(P, l, tot, nh, nc, st);
       if (r == TRY_STOPPED) active = false;
       if (r == TRY_ACCEPTED)
         while (l.cur + njobs < P.nsave && t_le<PR>(P.saveat[l.cur + njobs], l.t)) ++njobs;
@@ -2050,7 +2233,7 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P) {
     qcount += total < space ? total : space;
     (void)GBODE_CHECK(P, qcount >= 0 && qcount <= CAP, CHK_RING);
     if (r == TRY_ACCEPTED) {
-      adaptive_commit<M>(l, nh, nc);
+      adaptive_commit<MM>(l, nh, nc);
       store_step<PR, D>(P, l, l.nacc);
       if (!t_lt<PR>(l.t, P.tf)) {
         lane_finish(P, l, RET_DEFAULT, tot);
@@ -2289,22 +2472,29 @@ __device__ __forceinline__ void run_adaptive_staged2(const KParams& P) {
  * driver otherwise (large states: Verner 9 with dim 4, Kuramoto-12). */
 template <class M, class PR, int D, class F>
 __device__ __forceinline__ void run_adaptive_staged_or_persistent(const KParams& P) {
-  if constexpr (M::DENSE_F) {
-    /* dense output with extra stages: the two-queue form shares them between a step's save points */
-    if constexpr (StageLayout2<M, PR, D, F>::CR >= 32) {
-      if (P.nsave > 0) {
-        run_adaptive_staged2<M, PR, D, F>(P);
-        return;
-      }
-    }
-  }
-  if constexpr (StageLayout<M, PR, D, F>::CAP >= 32) {
+  /* dense output with extra stages: the two-queue form shares them between a step's save points */
+  constexpr bool two = M::DENSE_F && StageLayout2<M, PR, D, F>::CR >= 32, one = StageLayout<M, PR, D, F>::CAP >= 32;
+  constexpr int RING = two || one ? kStageBytesPerWarp : 0;
+  __shared__ typename PR::R kmem[kWarpsPerBlock][StageTypes<Stages<M, PR, D, F, RING>::SHARED, M, PR, D, F>::SLICE];
+  typename PR::R* slice = kmem[threadIdx.x >> 5];
+  if constexpr (two) {
     if (P.nsave > 0) {
-      run_adaptive_staged<M, PR, D, F>(P);
+      run_adaptive_staged2<M, PR, D, F>(P);
+      return;
+    }
+  } else if constexpr (one) {
+    if (P.nsave > 0) {
+      run_adaptive_staged<M, PR, D, F>(P, slice);
       return;
     }
   }
-  run_adaptive_persistent<M, PR, D, F>(P);
+  run_adaptive_persistent<M, PR, D, F, RING>(P, slice);
+}
+
+template <class M, class PR, int D, class F>
+__device__ __forceinline__ void run_adaptive_unstaged(const KParams& P) {
+  __shared__ typename PR::R kmem[kWarpsPerBlock][StageTypes<Stages<M, PR, D, F, 0>::SHARED, M, PR, D, F>::SLICE];
+  run_adaptive_persistent<M, PR, D, F, 0>(P, kmem[threadIdx.x >> 5]);
 }
 
 /* ------------------------------------------------------------------ fixed-step Tsit5, components over warps */
@@ -2548,7 +2738,7 @@ __device__ __forceinline__ void run_onestep(const KParams& P) {
   }
 #define GBODE_ENTRY_persistent(NAME, M, PR, RHS)                                             \
   extern "C" __global__ void __launch_bounds__(GBODE_BLOCK) NAME(gbode::KParams P) {                \
-    gbode::run_adaptive_persistent<M<PR, RHS::D, RHS>, PR, RHS::D, RHS>(P);                 \
+    gbode::run_adaptive_unstaged<M<PR, RHS::D, RHS>, PR, RHS::D, RHS>(P);                   \
   }
 #define GBODE_ENTRY_staged(NAME, M, PR, RHS)                                                 \
   extern "C" __global__ void __launch_bounds__(GBODE_BLOCK) NAME(gbode::KParams P) {                \
