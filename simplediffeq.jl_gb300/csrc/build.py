@@ -106,6 +106,7 @@ def gen_sources():
                        ("log_table.h", "kSrc_log_table_h"), ("exp_table.h", "kSrc_exp_table_h"),
                        ("ds_table.h", "kSrc_ds_table_h"), ("bitops.h", "kSrc_bitops_h"),
                        ("intchain.h", "kSrc_intchain_h"), ("introws.h", "kSrc_introws_h"),
+                       ("intpoly.h", "kSrc_intpoly_h"),
                        ("crpow.h", "kSrc_crpow_h"), ("crpow_table.h", "kSrc_crpow_table_h")):
         text = open(os.path.join(HERE, fname)).read()
         assert ")GBSRC\"" not in text
@@ -169,7 +170,7 @@ def build(verbose=False, jobs=None):
     os.makedirs(LIB, exist_ok=True)
     headers = [os.path.join(HERE, f) for f in ("ode_solver.cuh", "ode_kparams.h", "tableaus.h", "ode_host.h",
                                                "jlrange.h", "sde_solver.cuh", "log_table.h", "exp_table.h",
-                                               "ds_table.h", "bitops.h", "intchain.h", "introws.h", "crpow.h",
+                                               "ds_table.h", "bitops.h", "intchain.h", "introws.h", "intpoly.h", "crpow.h",
                                                "crpow_table.h")] + [
         os.path.join(PKG, "..", "include", "gb300ode.h")]
     host_tus = [os.path.join(HERE, f) for f in ("ode_capi.cu", "learn.cu", "noalloc.cu", "sde_capi.cu")]

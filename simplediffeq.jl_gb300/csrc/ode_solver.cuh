@@ -56,6 +56,7 @@
 #include "ode_kparams.h"
 #include "bitops.h"
 #include "introws.h"
+#include "intpoly.h"
 #ifdef GBODE_REF
 #include "crpow.h"
 #endif
@@ -87,19 +88,20 @@ __device__ __forceinline__ double sqrtR(double x) { return __dsqrt_rn(x); }
 __device__ __forceinline__ float sqrtR(float x) { return __fsqrt_rn(x); }
 __device__ __forceinline__ double absR(double x) { return fabs(x); }
 __device__ __forceinline__ float absR(float x) { return fabsf(x); }
-/* Sine and cosine of a double with one argument reduction, in 18 double
- * operations.  Method: Cody and Waite's reduction modulo pi/2 (W. J. Cody and
- * W. Waite, Software Manual for the Elementary Functions, 1980) in its fused
- * form: k = x * 2/pi rounded to the nearest integer (one fused multiply-add
- * with 1.5 * 2^52, whose low bits then hold k), r = (x - k*C1) - k*C2 with
- * C1 = pi/2 rounded to double and C2 the rounded remainder, each term one
- * fused multiply-add; then sin r = r + r^3 P(r^2) and cos r = 1 + r^2 Q(r^2)
- * with near-minimax P and Q of degree 5 from csrc/gen_sincos.py, in Horner
- * form.  Within 1.5 ulp (1.7e-16 absolute) of the exact values below 2^19
- * (checked against 40-digit values), except that results below 1e-15 in
- * magnitude (x within 1e-15 of a multiple of pi/2) keep an absolute error
- * below 1e-30 instead of a relative one.  Every step is one IEEE double operation, so the oracle reproduces it
- * bit for bit.  |x| >= 2^19 and non-finite x go to CUDA's sincos. */
+/* Sine and cosine of a double with one argument reduction.  Method: Cody and
+ * Waite's reduction modulo pi/2 (W. J. Cody and W. Waite, Software Manual for
+ * the Elementary Functions, 1980) in its fused form: k = x * 2/pi rounded to
+ * the nearest integer (one fused multiply-add with 1.5 * 2^52, whose low bits
+ * then hold k), r = (x - k*C1) - k*C2 with C1 = pi/2 rounded to double and C2
+ * the rounded remainder, each term one fused multiply-add; then sin r = r +
+ * r^3 P(r^2) and cos r = 1 + r^2 Q(r^2) with near-minimax P and Q of degree 5
+ * from csrc/gen_sincos.py, in Horner form.  Within 1.5 ulp (1.7e-16 absolute)
+ * of the exact values below 2^19 (checked against 40-digit values), except
+ * that results below 1e-15 in magnitude (x within 1e-15 of a multiple of
+ * pi/2) keep an absolute error below 1e-30 instead of a relative one.  Every
+ * step is one IEEE double operation or its bits (ip_sincos: eleven of the
+ * eighteen on the integer pipe), so the oracle reproduces it bit for bit.
+ * |x| >= 2^19 and non-finite x go to CUDA's sincos. */
 __device__ __forceinline__ void sincos_cw(double x, double* s, double* c) {
   /* |x| < 2^19 as an integer compare of the magnitude bits (a double compare
    * would issue on the FP64 pipe; NaN's bits lie above 2^19's, as its IEEE
@@ -114,20 +116,25 @@ __device__ __forceinline__ void sincos_cw(double x, double* s, double* c) {
   double r = __fma_rn(-k, 0x1.921fb54442d18p+0, x);
   r = __fma_rn(-k, 0x1.1a62633145c07p-54, r);
   const double z = r * r;
-  double ps = 0x1.5d8fd0a40698ep-33;
-  ps = __fma_rn(ps, z, -0x1.ae5e5a8d61ce7p-26);
-  ps = __fma_rn(ps, z, 0x1.71de3567ccfe8p-19);
-  ps = __fma_rn(ps, z, -0x1.a01a019bfde60p-13);
-  ps = __fma_rn(ps, z, 0x1.111111110f7d0p-7);
-  ps = __fma_rn(ps, z, -0x1.5555555555548p-3);
-  const double sr = __fma_rn(z * r, ps, r);
-  double pc = 0x1.1b8b9800ee7dap-29;
-  pc = __fma_rn(pc, z, -0x1.27df4604d6713p-22);
-  pc = __fma_rn(pc, z, 0x1.a019f81ca810ap-16);
-  pc = __fma_rn(pc, z, -0x1.6c16c1640a98bp-10);
-  pc = __fma_rn(pc, z, 0x1.555555554f0a9p-5);
-  pc = __fma_rn(pc, z, -0x1.fffffffffff96p-2);
-  const double cr = __fma_rn(z, pc, 1.0);
+  const double zr = z * r;
+  /* the polynomials: their eleven Horner steps run on the integer pipe */
+  double ps, cr;
+  if (__builtin_expect(!ip_sincos(z, &ps, &cr), 0)) {
+    ps = GBODE_SIN_C0;
+    ps = __fma_rn(ps, z, GBODE_SIN_C1);
+    ps = __fma_rn(ps, z, GBODE_SIN_C2);
+    ps = __fma_rn(ps, z, GBODE_SIN_C3);
+    ps = __fma_rn(ps, z, GBODE_SIN_C4);
+    ps = __fma_rn(ps, z, GBODE_SIN_C5);
+    double pc = GBODE_COS_C0;
+    pc = __fma_rn(pc, z, GBODE_COS_C1);
+    pc = __fma_rn(pc, z, GBODE_COS_C2);
+    pc = __fma_rn(pc, z, GBODE_COS_C3);
+    pc = __fma_rn(pc, z, GBODE_COS_C4);
+    pc = __fma_rn(pc, z, GBODE_COS_C5);
+    cr = __fma_rn(z, pc, 1.0);
+  }
+  const double sr = __fma_rn(zr, ps, r);
   /* quadrant q: (sin, cos) = (sr, cr), (cr, -sr), (-sr, -cr), (-cr, sr); the
    * negations flip the sign bit of the high word, off the FP64 pipe */
   const double so = (q & 1) ? cr : sr, co = (q & 1) ? sr : cr;
@@ -754,26 +761,45 @@ struct RhsR3BP {
   }
 };
 
-/* The phases' sine/cosine loop is kept rolled: unrolled, the seven right-hand
- * side evaluations of a Tsit5 step put 7 x 12 sine/cosine bodies in the step
- * loop, more code than the instruction cache holds once the warps of an SM
- * are at different points of their steps (measured on the persistent
- * kernel: about ten warps waiting for instruction fetch per instruction
- * issued, and 1.56x the time of a rolled loop).  Indexed by the loop
- * counter, the phases and the sines and cosines live in local memory (L1),
- * whose traffic costs far less than the FP64 work it sits between. */
+/* The phases' sine/cosine loop is kept rolled, and in double precision out of
+ * line: inlined and unrolled, the seven right-hand side evaluations of a Tsit5
+ * step put 7 x 12 sine/cosine bodies in the step loop, more code than the
+ * instruction cache holds once the warps of an SM are at different points of
+ * their steps (measured on the persistent kernel: about ten warps waiting for
+ * instruction fetch per instruction issued, and 1.56x the time of a rolled
+ * loop).  With the polynomials on the integer pipe a body is some 200
+ * instructions, and seven rolled copies of it already cost as much: 131,072
+ * Kuramoto-12 trajectories took 134.1 ms, and 91.2 ms with one copy (114.2 ms
+ * with multiply-add polynomials inline).  Indexed by the loop counter, the
+ * phases and the sines and cosines live in local memory (L1), whose traffic
+ * costs far less than the FP64 work it sits between. */
+/* sines and cosines of n phases and their sums, added in order */
+template <class R>
+__device__ __forceinline__ void phase_sums(int n, const R* u, R* sn, R* cs, R* So, R* Co) {
+  R S = 0, C = 0;
+#pragma unroll 1
+  for (int j = 0; j < n; ++j) {
+    sincosR(u[j], &sn[j], &cs[j]);
+    S = S + sn[j];
+    C = C + cs[j];
+  }
+  *So = S;
+  *Co = C;
+}
+static __device__ __noinline__ void phase_sums_once(int n, const double* u, double* sn, double* cs, double* So, double* Co) {
+  phase_sums<double>(n, u, sn, cs, So, Co);
+}
+static __device__ __forceinline__ void phase_sums_once(int n, const float* u, float* sn, float* cs, float* So, float* Co) {
+  phase_sums<float>(n, u, sn, cs, So, Co);
+}
+
 template <class R, class T, int DD>
 struct RhsKuramoto {
   enum { D = DD, NP = DD + 1 };
   R p[DD + 1];  /* omega_1..omega_D, then K / D (rhs_loaded divides the loaded K once) */
   __device__ __forceinline__ void operator()(const R (&u)[DD], T t, R (&du)[DD]) const {
-    R sn[DD], cs[DD], S = 0, C = 0;
-#pragma unroll 1
-    for (int j = 0; j < DD; ++j) {
-      sincosR(u[j], &sn[j], &cs[j]);
-      S = S + sn[j];
-      C = C + cs[j];
-    }
+    R sn[DD], cs[DD], S, C;
+    phase_sums_once(DD, u, sn, cs, &S, &C);
     const R kd = p[DD];
 #pragma unroll
     for (int i = 0; i < DD; ++i) {
