@@ -64,11 +64,13 @@ GROUPS = {
     "kuramoto": [("atsit5", "plain", "kuramoto", 12, "fp64"),
                  ("atsit5", "persistent", "kuramoto", 12, "fp64")],
     "kuramoto_staged": [("atsit5", "staged", "kuramoto", 12, "fp64")],
-    # the same with the stages' linear combinations on the integer pipe, for ensembles that fill the GPU
-    # (use_integer_pipe in ode_capi.cu)
-    "lorenz_ic": [("atsit5", "plain", "lorenz", 3, "fp64"),
+    # the same for ensembles that crowd the GPU (crowded() in ode_capi.cu)
+    "lorenz_crowded": [("atsit5", "plain", "lorenz", 3, "fp64"),
                   ("atsit5", "persistent", "lorenz", 3, "fp64")],
-    "lorenz_staged_ic": [("atsit5", "staged", "lorenz", 3, "fp64")],
+    "lorenz_staged_crowded": [("atsit5", "staged", "lorenz", 3, "fp64")],
+    "kuramoto_crowded": [("atsit5", "plain", "kuramoto", 12, "fp64"),
+                         ("atsit5", "persistent", "kuramoto", 12, "fp64")],
+    "kuramoto_staged_crowded": [("atsit5", "staged", "kuramoto", 12, "fp64")],
 }
 
 
@@ -77,17 +79,17 @@ GROUPS = {
 # shape the autotuner picks on the benchmark workloads (a ring that holds a
 # round plus a step's worth of new jobs, at no cost in occupancy); Kuramoto-12's
 # 804-byte jobs take one-warp blocks with a ring of exactly one round (32 jobs),
-# eight warps per SM.  The integer-pipe kernel's warps also hold their stages in
+# eight warps per SM.  The crowded GPU's Lorenz kernel's warps also hold their stages in
 # shared memory, and it gains from every warp there is room for: the smallest
 # rings (36 jobs) in two-warp blocks give 16 warps per SM (1M learned Lorenz
 # solve: 104.8 ms with 8 warps per SM, 92.5 with 10, 84.6 with 12, 80.5 with 14,
 # 77.1 with 16).
 SHAPES = {"lorenz_staged": (64, 24576), "vdp_staged": (64, 24576), "kuramoto_staged": (32, 26112),
-          "lorenz_staged_ic": (64, 8704)}
+          "lorenz_staged_crowded": (64, 8704), "kuramoto_staged_crowded": (32, 26112)}
 
 
-def kname(alg, kind, rhs, dim, prec, ic=False):
-    return "gbode_%s_%s_%s%d_%s%s" % (alg, kind, rhs, dim, prec, "_ic" if ic else "")
+def kname(alg, kind, rhs, dim, prec, crowded=False):
+    return "gbode_%s_%s_%s%d_%s%s" % (alg, kind, rhs, dim, prec, "_crowded" if crowded else "")
 
 
 def write_if_changed(path, text):
@@ -116,26 +118,26 @@ def gen_sources():
     decl, entries, tus = [], [], []
     for g, items in GROUPS.items():
         block, ring = SHAPES.get(g, (128, 12288))
-        ic = g.endswith("_ic")
+        crowded = g.endswith("_crowded")
         lines = ["/* generated by build.py: ahead-of-time kernels, group %s */\n" % g,
                  "#define GBODE_BLOCK %d\n#define GBODE_STAGE_BYTES %d\n" % (block, ring),
                  "#define GBODE_CTRL_DS 1 /* the default error norm and controller (ODE_CTRL_DS) */\n",
-                 "#define GBODE_IC 1\n" if ic else "",
+                 "#define GBODE_CROWDED 1\n" if crowded else "",
                  '#include "ode_solver.cuh"\n']
         for i, (alg, kind, rhs, dim, prec) in enumerate(items):
             t = "RHS_%s_%d" % (g, i)
             lines.append("typedef %s %s;\n" % (rhs_type(rhs, dim, prec), t))
-            lines.append("GBODE_ENTRY(%s, %s, %s, %s, %s)\n" % (kname(alg, kind, rhs, dim, prec, ic), kind,
+            lines.append("GBODE_ENTRY(%s, %s, %s, %s, %s)\n" % (kname(alg, kind, rhs, dim, prec, crowded), kind,
                                                                METHOD[alg], PREC[prec][1], t))
-            decl.append('extern "C" __global__ void %s(gbode::KParams);\n' % kname(alg, kind, rhs, dim, prec, ic))
+            decl.append('extern "C" __global__ void %s(gbode::KParams);\n' % kname(alg, kind, rhs, dim, prec, crowded))
             entries.append('  {%d, "%s", %d, %d, %d, (const void*)%s, %d, %d, %d},\n' % (
-                ALG[alg], kind, RHS[rhs], dim, PREC[prec][0], kname(alg, kind, rhs, dim, prec, ic), block, ring, int(ic)))
+                ALG[alg], kind, RHS[rhs], dim, PREC[prec][0], kname(alg, kind, rhs, dim, prec, crowded), block, ring, int(crowded)))
         path = os.path.join(BUILD, "kern_%s.cu" % g)
         write_if_changed(path, "".join(lines))
         tus.append(path)
     reg = ["/* generated by build.py: kernels compiled ahead of time */\n",
            "struct AotEntry { int alg; const char* kind; int rhs; int dim; int precision; const void* fn; int block; "
-           "int stage; int ic; };\n"]
+           "int stage; int crowded; };\n"]
     reg += decl
     reg.append("static const AotEntry kAotEntries[] = {\n")
     reg += entries

@@ -337,9 +337,21 @@ int stage_slice_bytes(const ode_solve_args* a) { return 7 * a->dim * 32 * 8; }
 /* A ring of 36 units, in steps of 512 bytes: a round of 32 and a few more. */
 int small_ring_bytes(const ode_solve_args* a) { return (36 * stage_unit_bytes(a) + 511) / 512 * 512; }
 
-/* Whether this solve runs the kernel that keeps the stages in shared memory
- * and forms their linear combinations on the integer pipe (GBODE_IC,
- * intchain.h): adaptive Tsit5 in FP64, in the default rounding.
+/* Whether the ensemble crowds the GPU: more than two warps of trajectories for
+ * every SM sub-partition (38,912).  Adaptive Tsit5 in FP64 and the default
+ * rounding has kernels of its own for that (GBODE_CROWDED): their warps merge
+ * when the ensemble runs out (Feed), and where they fit they run linear
+ * combinations on the integer pipe.  The smaller ensembles' kernels do
+ * without the code for it, whose few instructions an attempt cost a lone
+ * trajectory 0.6%. */
+bool crowded(const ode_handle* h, const ode_solve_args* a) {
+  if (a->alg != ODE_ALG_ATSIT5 || a->precision != ODE_FP64 || a->controller == ODE_CTRL_REF) return false;
+  if (h->tune_crowded >= 0) return h->tune_crowded != 0;
+  return a->n > (int64_t)h->nsm * 4 * 64;
+}
+
+/* Whether its kernel keeps the stages in shared memory and forms their linear
+ * combinations on the integer pipe (Stages<...>::SHARED, intchain.h).
  *
  * It pays once the FP64 pipe is shared.  A lone warp waits as long for a
  * linear combination of integers as for one of fused multiply-adds; with more
@@ -351,15 +363,11 @@ int small_ring_bytes(const ode_solve_args* a) { return (36 * stage_unit_bytes(a)
  *   Lotka-Volterra, saveat   0.95    0.94    1.12    1.04    1.08
  *   linear, dim 4, saveat    1.05    1.05    1.08    1.06    1.23
  *   linear, dim 6            1.03    1.04    1.04    1.05    1.15
- * (two warps on each of the 608 sub-partitions are 38,912 trajectories).  The
- * size limit keeps at least 12 warps an SM: with fewer the integer pipe's
+ * The size limit keeps at least 12 warps an SM: with fewer the integer pipe's
  * latency shows (the Lorenz solve above at 8: no gain). */
 bool use_integer_pipe(const ode_handle* h, const ode_solve_args* a, int sched) {
-  if (a->alg != ODE_ALG_ATSIT5 || a->precision != ODE_FP64 || a->controller == ODE_CTRL_REF) return false;
   const bool staged = !std::strcmp(entry_kind(a->alg, sched, a->nsave), "staged");
-  if (stage_slice_bytes(a) + (staged ? small_ring_bytes(a) : 0) > 19456) return false;
-  if (h->tune_int >= 0) return h->tune_int != 0;
-  return a->n > (int64_t)h->nsm * 4 * 64;
+  return crowded(h, a) && stage_slice_bytes(a) + (staged ? small_ring_bytes(a) : 0) <= 19456;
 }
 
 /* Launch shape of an untuned run-time compiled kernel: 128 threads and 12 KB
@@ -415,7 +423,7 @@ std::string kernel_key(ode_handle* h, const ode_solve_args* a, int sched) {
   char b[160];
   snprintf(b, sizeof b, "%s|%s|%d|%d|%s|%d%s%s%s", alg_name(a->alg), kernel_kind(h, a, sched), a->rhs, a->dim,
            prec_name(a->precision), a->output >= ODE_OUTPUT_USER ? a->output : 0, h->bounds_check ? "|chk" : "",
-           ctrl_suffix(ctrl_variant(a)), use_integer_pipe(h, a, sched) ? "|ic" : "");
+           ctrl_suffix(ctrl_variant(a)), crowded(h, a) ? "|crowded" : "");
   return b;
 }
 
@@ -423,7 +431,7 @@ std::string kernel_key(ode_handle* h, const ode_solve_args* a, int sched) {
  * dim, schedule kind). */
 std::string jit_source(ode_handle* h, const ode_solve_args* a, int sched) {
   std::string src;
-  if (use_integer_pipe(h, a, sched)) src += "#define GBODE_IC 1\n";
+  if (crowded(h, a)) src += "#define GBODE_CROWDED 1\n";
   if (ctrl_variant(a) == ODE_CTRL_FP64) src += "#define GBODE_CTRL64 1\n";
   if (ctrl_variant(a) == ODE_CTRL_DS) src += "#define GBODE_CTRL_DS 1\n";
   if (ctrl_variant(a) == ODE_CTRL_REF) src += "#define GBODE_REF 1\n";
@@ -560,12 +568,12 @@ int get_kernel(ode_handle* h, const ode_solve_args* a, int sched, CUfunction* fn
     return ODE_OK;
   }
   const char* kind = kernel_kind(h, a, sched);
-  const bool ic = use_integer_pipe(h, a, sched);
+  const bool crowd = crowded(h, a);
   for (const AotEntry& e : kAotEntries) {
     if (!h->bounds_check && ctrl_variant(a) == ODE_CTRL_DS && a->output < ODE_OUTPUT_USER && e.alg == a->alg &&
         e.rhs == a->rhs &&
         e.dim == a->dim &&
-        e.precision == a->precision && std::strcmp(e.kind, kind) == 0 && (e.ic != 0) == ic) {
+        e.precision == a->precision && std::strcmp(e.kind, kind) == 0 && (e.crowded != 0) == crowd) {
       cudaFunction_t f;
       cudaError_t ce = cudaGetFuncBySymbol(&f, e.fn);
       if (ce != cudaSuccess) return cuda_fail(h, ce, "cudaGetFuncBySymbol");
@@ -674,14 +682,14 @@ static std::string gpu_tag(ode_handle* h) {
   return name + "/" + std::to_string(prop.multiProcessorCount);
 }
 
-/* kernel keys are alg|kind|rhs|dim|prec|output[|chk][|c64, |c32 or |ref][|ic]; only built-in ids travel,
+/* kernel keys are alg|kind|rhs|dim|prec|output[|chk][|c64, |c32 or |ref][|crowded]; only built-in ids travel,
  * and no bounds-check build */
 static bool portable_key(const std::string& key) {
   std::vector<std::string> f;
   size_t a = 0;
   for (size_t b; (b = key.find('|', a)) != std::string::npos; a = b + 1) f.push_back(key.substr(a, b - a));
   f.push_back(key.substr(a));
-  if (f.size() > 6 && f.back() == "ic") f.pop_back();
+  if (f.size() > 6 && f.back() == "crowded") f.pop_back();
   const bool has_ctrl = f.size() == 7 && (f[6] == "c64" || f[6] == "c32" || f[6] == "ref");
   return (f.size() == 6 || has_ctrl) && std::atoi(f[2].c_str()) < ODE_RHS_USER &&
          std::atoi(f[5].c_str()) < ODE_OUTPUT_USER;
@@ -1083,6 +1091,19 @@ int solve_impl(ode_handle* h, const ode_solve_args* a, ode_solve_out* o, ode_sol
     gridx = (unsigned)std::max<int64_t>(1, std::min<int64_t>(resident, (n + block - 1) / block));
   }
 
+  /* the place where the persistent kernels' warps park trajectories to merge (Feed in ode_solver.cuh) */
+  int* park_ctl = nullptr;
+  size_t park_bytes = 0;
+  if (sched != ODE_SCHED_PLAIN && crowded(h, a)) {
+    const size_t cap = (size_t)gridx * block;
+    park_bytes = (PARK_FLAGS + cap) * sizeof(int);
+    if (!(park_ctl = (int*)buf(h, nm("park_ctl"), park_bytes, &rc))) return rc;
+    if (!(kp.park = (double*)buf(h, nm("park"), cap * park_words(D) * sizeof(double), &rc))) return rc;
+    kp.park_ctl = park_ctl;
+    kp.park_cap = (long long)cap;
+    kp.park_min = kp.park_slots = h->nsm * 4;
+  }
+
   /* device buffers of the learned schedule, allocated before any capture */
   float *latt = nullptr, *ldt = nullptr;
   int* order = nullptr;
@@ -1104,6 +1125,7 @@ int solve_impl(ode_handle* h, const ode_solve_args* a, ode_solve_out* o, ode_sol
    * graph and replayed while the launch parameters stay the same. */
   auto enqueue = [&](int* nl) -> int {
     CK(cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), s), "memset stats");
+    if (park_ctl) CK(cudaMemsetAsync(park_ctl, 0, park_bytes, s), "memset parking");
     if (chk) CK(cudaMemsetAsync(chk, 0, ((size_t)n + 16) * sizeof(unsigned), s), "memset check");
     if (sched == ODE_SCHED_LEARNED && n > 0) {
       int r = model_predict_device(h, a, kp, latt, ldt, s, nl);
@@ -1626,11 +1648,11 @@ int ode_autotune(ode_handle* h, const ode_solve_args* a, int64_t sample, ode_tun
   to.us = dus;
   to.u_final = duf;
   /* the whole ensemble's kernel is tuned, whatever the sample's size would choose */
-  struct TuneInt {
+  struct TuneCrowded {
     ode_handle* h;
-    ~TuneInt() { h->tune_int = -1; }
-  } tune_int{h};
-  h->tune_int = use_integer_pipe(h, a, ta.schedule);
+    ~TuneCrowded() { h->tune_crowded = -1; }
+  } tune_crowded{h};
+  h->tune_crowded = crowded(h, a);
   const bool ic = use_integer_pipe(h, &ta, ta.schedule);
   const std::string key = kernel_key(h, &ta, ta.schedule);
   /* the baseline is the kernel an untuned handle would run */

@@ -10,6 +10,15 @@ namespace gbode {
 
 enum { RET_DEFAULT = 0, RET_DTMIN = 1, RET_MAXITERS = 2, RET_NAN = 3 };
 
+/* Words of the parking place (Feed in ode_solver.cuh): lanes without work less
+ * the parked trajectories, warps at work, entries written, entries taken; from
+ * PARK_SLOTS on the warps at work on each sub-partition, from PARK_FLAGS on a
+ * flag per entry that its trajectory is there. */
+enum { PARK_IDLE = 0, PARK_WARPS = 1, PARK_TAIL = 2, PARK_HEAD = 3, PARK_SLOTS = 16, PARK_MAX_SLOTS = 1024,
+       PARK_FLAGS = PARK_SLOTS + PARK_MAX_SLOTS };
+/* doubles of a parked trajectory of dimension D: at most three per component and 12 */
+constexpr int park_words(int D) { return 3 * D + 12; }
+
 struct KParams {
   long long n;             /* trajectories */
   double t0, tf, dt, abstol, reltol;
@@ -40,6 +49,11 @@ struct KParams {
   double* ev_u;            /* [rows][dim] state after each accepted step (u0 first) */
   const int* order;        /* persistent: position -> trajectory, or 0 for identity */
   unsigned long long* counter;   /* persistent: next position to hand out (zeroed before launch) */
+  int* park_ctl;           /* persistent: the parking place's words (ParkWord, then the sub-partitions' warp
+                              counts and the entries' flags; zeroed before launch), or 0: no parking */
+  double* park;            /* [PARK_WORDS][park_cap] parked trajectories */
+  long long park_cap;      /* entries: the launch's lanes */
+  int park_min, park_slots; /* warps below which none parks; SM sub-partitions */
   unsigned long long* stats;     /* [2] attempts and saves summed over trajectories, or 0 */
   unsigned* check_flags;   /* bounds-check builds: violation bits (CHK_*), or 0 */
   unsigned* visited;       /* bounds-check builds: [n] starts of each trajectory, or 0 */

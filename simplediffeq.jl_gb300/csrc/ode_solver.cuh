@@ -1420,17 +1420,21 @@ struct MInt : M {
   }
 };
 
+/* The kernels for ensembles that crowd the GPU (crowded() in ode_capi.cu). */
+#if defined(GBODE_CROWDED) && !defined(GBODE_REF)
+enum { CROWDED = 1 };
+#else
+enum { CROWDED = 0 };
+#endif
+
 /* Whether the adaptive kernels of this method and size keep the stages in
  * shared memory and run their linear combinations on the integer pipe, and
  * the types that follow from it.  RING: the staging ring's bytes per warp. */
 template <class M, class PR, int D, class F, int RING>
 struct Stages {
   enum { BYTES = M::NK * D * 32 * 8 };
-#if defined(GBODE_IC) && !defined(GBODE_REF)
-  enum { SHARED = M::IC && sizeof(typename PR::R) == 8 && (GBODE_BLOCK / 32) * (BYTES + RING) <= 49152 };
-#else
-  enum { SHARED = 0 };
-#endif
+  enum { SHARED = CROWDED && M::IC && sizeof(typename PR::R) == 8 && BYTES + RING <= 19456 &&
+                  (GBODE_BLOCK / 32) * (BYTES + RING) <= 49152 };
 };
 template <bool SHARED, class M, class PR, int D, class F> struct StageTypes {
   typedef M Method;
@@ -2036,22 +2040,137 @@ __device__ __forceinline__ void run_adaptive_plain(const KParams& P) {
   flush_totals(P, tot);
 }
 
-/* Persistent schedule: resident warps loop over attempts; a lane whose
- * trajectory finished takes the next position from a device counter
- * (one atomicAdd per warp for all lanes that need work) and the position is
- * mapped through P.order.  Every lane of a warp runs the loop until the whole
- * warp has no work left, so the warp-wide ballots stay convergent. */
-template <class M, class PR, int D, class F, int RING>
-__device__ __forceinline__ void run_adaptive_persistent(const KParams& P, typename PR::R* slice) {
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  typedef StageTypes<Stages<M, PR, D, F, RING>::SHARED, M, PR, D, F> ST;
-  typedef typename ST::Method MM;
-  Lane<PR, D, F, M::NK, typename ST::KS> l;
-  ST::bind(l.k, slice);
-  Totals tot = {0, 0, 0};
-  bool active = false, exhausted = false;
-  for (;;) {
+/* ------------------------------------------------------------------ work for the persistent schedules */
+/* A trajectory between two attempts, to and from entry i of the parking place
+ * (past L1: another SM reads it).  Parameters are loaded again. */
+template <class PR, int D, class F, int NK, class KS, bool FSAL>
+__device__ __forceinline__ void lane_park(const KParams& P, Lane<PR, D, F, NK, KS>& l, long long i) {
+  double* e = P.park + i;
+  const long long c = P.park_cap;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    __stcg(e, (double)l.uh[d]); e += c;
+    if (PR::KAHAN) { __stcg(e, (double)l.uc[d]); e += c; }
+    if (FSAL) { __stcg(e, (double)l.k[0][d]); e += c; }
+  }
+  __stcg(e, (double)l.t); e += c;
+  __stcg(e, (double)l.dt); e += c;
+  __stcg(e, l.dt_first); e += c;
+  __stcg(e, __longlong_as_double(l.idx)); e += c;
+  __stcg(e, __longlong_as_double(l.att)); e += c;
+  __stcg(e, __longlong_as_double(l.cur)); e += c;
+  __stcg(e, __longlong_as_double(l.ninterp)); e += c;
+  __stcg(e, __hiloint2double(l.nacc, l.nrej)); e += c;
+  __stcg(e, __hiloint2double(l.nan_seen ? 1 : 0, __float_as_int(l.qoldp))); e += c;
+#ifdef GBODE_CTRL_DS
+  __stcg(e, __hiloint2double(__float_as_int(l.lqds.h), __float_as_int(l.lqds.l))); e += c;
+#endif
+#ifdef GBODE_CTRL64
+  __stcg(e, l.lqold); e += c;
+#endif
+#ifdef GBODE_REF
+  __stcg(e, l.qold); e += c;
+#endif
+}
+template <class PR, int D, class F, int NK, class KS, bool FSAL>
+__device__ __forceinline__ void lane_unpark(const KParams& P, Lane<PR, D, F, NK, KS>& l, long long i) {
+  typedef typename PR::R R;
+  typedef typename PR::T T;
+  const double* e = P.park + i;
+  const long long c = P.park_cap;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    l.uh[d] = (R)__ldcg(e); e += c;
+    l.uc[d] = (R)0;
+    if (PR::KAHAN) { l.uc[d] = (R)__ldcg(e); e += c; }
+    if (FSAL) { l.k[0][d] = (R)__ldcg(e); e += c; }
+  }
+  l.t = (T)__ldcg(e); e += c;
+  l.dt = (T)__ldcg(e); e += c;
+  l.dt_first = __ldcg(e); e += c;
+  l.idx = __double_as_longlong(__ldcg(e)); e += c;
+  l.att = __double_as_longlong(__ldcg(e)); e += c;
+  l.cur = __double_as_longlong(__ldcg(e)); e += c;
+  l.ninterp = __double_as_longlong(__ldcg(e)); e += c;
+  double w = __ldcg(e); e += c;
+  l.nacc = __double2hiint(w);
+  l.nrej = __double2loint(w);
+  w = __ldcg(e); e += c;
+  l.nan_seen = __double2hiint(w) != 0;
+  l.qoldp = __int_as_float(__double2loint(w));
+#ifdef GBODE_CTRL_DS
+  w = __ldcg(e); e += c;
+  l.lqds = {__int_as_float(__double2hiint(w)), __int_as_float(__double2loint(w))};
+#endif
+#ifdef GBODE_CTRL64
+  l.lqold = __ldcg(e); e += c;
+#endif
+#ifdef GBODE_REF
+  l.qold = __ldcg(e); e += c;
+#endif
+#pragma unroll
+  for (int j = 0; j < F::NP; ++j) l.f.p[j] = (R)P.p[(long long)j * P.n + l.idx];
+  rhs_loaded(l.f);
+}
+
+/* Hands a warp's lanes their trajectories.  While the device counter has
+ * positions left, a lane that finished takes the next one (one atomicAdd per
+ * warp for all lanes that need work), mapped through P.order.
+ *
+ * After that, in the kernels for crowded GPUs, lanes run out of work one by one, and a warp instruction costs
+ * the same with one lane at work as with 32 (the FP64 pipe takes 64 cycles
+ * either way): of 100,000 Lorenz trajectories on 78,000 lanes, 19.5 lanes of a
+ * warp were at work on average.  So warps merge: when 32 lanes over all warps
+ * are without work, a warp parks its trajectories in global memory and ends,
+ * and lanes without work take them up.  PARK_IDLE counts those lanes less the
+ * parked trajectories, and a warp takes 32 of them (its own and one for each
+ * trajectory it parks) before it parks, so no more are parked than can be
+ * taken up.  Merging stops at one warp per sub-partition, where a warp has its
+ * pipe to itself.  Only warps on sub-partitions with at least the average
+ * number of warps park: whichever warp came first, the sub-partitions lost
+ * balance and the solve above took 14.7 ms (11.9 without merging, 10.4 as it
+ * is).  A warp looks once in 16 attempts: a look takes an L2 round trip, and
+ * the emptier the warps get meanwhile, the fewer move (each attempt 11.8 ms,
+ * once in 4 11.4, in 8 10.9, in 32 10.6, in 64 10.9).  Others: 131,072
+ * Kuramoto-12 87.1 to 83.2 ms, 200,003 Van der Pol 34.5 to 33.8, 65,536 single-
+ * precision three-body 26.6 to 25.9, 100,003 Lorenz final states 11.5 to 9.7.
+ *
+ * Nothing waits on another warp: entries are taken only once their flags are
+ * there, a warp out of work gives lanes that others count on a bounded number
+ * of polls, and the last warp to end (PARK_WARPS) looks once more, so a parked
+ * trajectory is always taken up. */
+struct Feed {
+  bool exhausted;   /* this lane found the counter at its end */
+  bool quiet;       /* no warp parks any more */
+  int counted;      /* lanes of this warp in PARK_IDLE */
+  int tick, polls;
+  int* slot;        /* the sub-partition's count of warps */
+
+  __device__ __forceinline__ void init(const KParams& P) {
+    exhausted = false;
+    quiet = false;
+    counted = 0;
+    tick = 0;
+    polls = 0;
+    slot = 0;
+    if (!CROWDED || !P.park_ctl) return;
+    unsigned sm, w;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    asm volatile("mov.u32 %0, %%warpid;" : "=r"(w));
+    /* a warp's sub-partition goes by its id */
+    slot = P.park_ctl + PARK_SLOTS + (int)((sm * 4u + (w & 3u)) % PARK_MAX_SLOTS);
+    slot = (int*)__shfl_sync(0xffffffffu, (unsigned long long)slot, 0);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(P.park_ctl + PARK_WARPS, 1);
+      atomicAdd(slot, 1);
+    }
+  }
+
+  /* true: go on (some lane may be active); false: the warp's work is done */
+  template <class M, class PR, int D, class F, int NK, class KS>
+  __device__ __forceinline__ bool next(const KParams& P, Lane<PR, D, F, NK, KS>& l, bool& active, Totals& tot) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
     const bool want = !active && !exhausted;
     const unsigned need = __ballot_sync(FULL, want);
     if (need) {
@@ -2064,16 +2183,134 @@ __device__ __forceinline__ void run_adaptive_persistent(const KParams& P, typena
         if (w < (unsigned long long)P.n) {
           long long idx = P.order ? (long long)P.order[w] : (long long)w;
           if (!GBODE_CHECK(P, idx >= 0 && idx < P.n, CHK_ORDER)) idx = 0;
-          active = !adaptive_start<MM>(P, idx, l, tot);
+          active = !adaptive_start<M>(P, idx, l, tot);
         } else {
           exhausted = true;
         }
       }
     }
-    if (!__any_sync(FULL, active)) {
-      if (!__any_sync(FULL, !exhausted)) break;
-      continue;
+    if (!CROWDED) return __any_sync(FULL, active) || __any_sync(FULL, !exhausted);
+    const unsigned act = __ballot_sync(FULL, active);
+    if (!__any_sync(FULL, exhausted)) return true;
+    if (!P.park_ctl) return act != 0 || __any_sync(FULL, !exhausted);
+
+    const int at_work = __popc(act), idle = 32 - at_work;
+    if (at_work > 0 && (quiet || (++tick & 15) != 0)) return true;
+    int* ctl = P.park_ctl;
+    int v = 0;
+    if (lane < 5) v = __ldcg(lane < 4 ? ctl + lane : slot);
+    int free_lanes = __shfl_sync(FULL, v, PARK_IDLE);
+    const int warps = __shfl_sync(FULL, v, PARK_WARPS), tail = __shfl_sync(FULL, v, PARK_TAIL);
+    const int head = __shfl_sync(FULL, v, PARK_HEAD), here = __shfl_sync(FULL, v, 4);
+    if (idle != counted) {
+      if (lane == 0) atomicAdd(ctl + PARK_IDLE, idle - counted);
+      free_lanes += idle - counted;
+      counted = idle;
     }
+    if (tail > head && idle > 0) {
+      const int most = tail - head < idle ? tail - head : idle;
+      int there = 0;
+      if (lane < most) there = __ldcg(ctl + PARK_FLAGS + head + lane);
+      const unsigned ready = __ballot_sync(FULL, there != 0);
+      const int take = ready == FULL ? 32 : __ffs(~ready) - 1;
+      int got = 0;
+      if (take > 0) {
+        if (lane == 0) got = atomicCAS(ctl + PARK_HEAD, head, head + take) == head;
+        got = __shfl_sync(FULL, got, 0);
+      }
+      if (got) {
+        __threadfence();
+        const int rank = __popc(~act & ((1u << lane) - 1u));
+        if (!active && rank < take) {
+          lane_unpark<PR, D, F, NK, KS, M::FSAL != 0>(P, l, head + rank);
+          active = true;
+        }
+        counted -= take;
+        return true;
+      }
+    } else if (at_work > 0 && free_lanes >= 32 && warps > P.park_min && (long long)here * P.park_slots >= warps) {
+      int room = 0, base = 0;
+      if (lane == 0) {
+        room = atomicSub(ctl + PARK_IDLE, 32) >= 32;
+        if (room) base = atomicAdd(ctl + PARK_TAIL, at_work);
+        else atomicAdd(ctl + PARK_IDLE, 32);
+      }
+      room = __shfl_sync(FULL, room, 0);
+      base = __shfl_sync(FULL, base, 0);
+      if (room) {
+        const int i = base + __popc(act & ((1u << lane) - 1u));
+        if (active) {
+          lane_park<PR, D, F, NK, KS, M::FSAL != 0>(P, l, i);
+          __threadfence();
+          __stcg(ctl + PARK_FLAGS + i, 1);
+          active = false;
+          exhausted = true;
+        }
+        counted = 0;
+        return leave(P, lane);
+      }
+    }
+    if (at_work > 0) {
+      quiet = warps <= P.park_min && tail == head;
+      return true;
+    }
+    /* no work: end, unless parked trajectories count on this warp's lanes */
+    int stay = 0;
+    if (lane == 0) {
+      const int before = atomicSub(ctl + PARK_IDLE, counted);
+      if (before < counted && polls < 256) {
+        atomicAdd(ctl + PARK_IDLE, counted);
+        stay = 1;
+      }
+    }
+    stay = __shfl_sync(FULL, stay, 0);
+    if (stay) {
+      ++polls;
+      __nanosleep(1000);
+      return true;
+    }
+    counted = 0;
+    return leave(P, lane);
+  }
+
+  /* the warp ends; true if it was the last one and trajectories are still parked */
+  __device__ __forceinline__ bool leave(const KParams& P, int lane) {
+    int again = 0;
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) {
+      int* ctl = P.park_ctl;
+      const bool last = atomicSub(ctl + PARK_WARPS, 1) == 1;
+      atomicSub(slot, 1);
+      __threadfence();
+      if (last && __ldcg(ctl + PARK_TAIL) > __ldcg(ctl + PARK_HEAD)) {
+        again = 1;
+        atomicAdd(ctl + PARK_WARPS, 1);
+        atomicAdd(slot, 1);
+      }
+    }
+    return __shfl_sync(0xffffffffu, again, 0) != 0;
+  }
+};
+
+/* Persistent schedule: resident warps loop over attempts, their lanes handed
+ * trajectories by Feed.  Every lane of a warp runs the loop until the whole
+ * warp has no work left, so the warp-wide ballots stay convergent. */
+template <class M, class PR, int D, class F, int RING>
+__device__ __forceinline__ void run_adaptive_persistent(const KParams& P, typename PR::R* slice) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  typedef StageTypes<Stages<M, PR, D, F, RING>::SHARED, M, PR, D, F> ST;
+  typedef typename ST::Method MM;
+  Lane<PR, D, F, M::NK, typename ST::KS> l;
+  ST::bind(l.k, slice);
+  Totals tot = {0, 0, 0};
+  bool active = false;
+  Feed feed;
+  feed.init(P);
+  for (;;) {
+    if (!feed.next<MM>(P, l, active, tot)) break;
+    if (!__any_sync(FULL, active)) continue;
     if (active && adaptive_iter<MM>(P, l, tot)) active = false;
   }
   flush_totals(P, tot);
@@ -2141,7 +2378,9 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P, typename P
   Lane<PR, D, F, NK, typename ST::KS> l;
   ST::bind(l.k, slice);
   Totals tot = {0, 0, 0};
-  bool active = false, exhausted = false;
+  bool active = false;
+  Feed feed;
+  feed.init(P);
 
   /* interpolate the m oldest jobs, one per lane */
   auto round = [&](int m) {
@@ -2174,28 +2413,8 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P, typename P
   };
 
   for (;;) {
-    const bool want = !active && !exhausted;
-    const unsigned need = __ballot_sync(FULL, want);
-    if (need) {
-      const int leader = __ffs(need) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(P.counter, (unsigned long long)__popc(need));
-      base = __shfl_sync(FULL, base, leader);
-      if (want) {
-        const unsigned long long w = base + (unsigned long long)__popc(need & ((1u << lane) - 1u));
-        if (w < (unsigned long long)P.n) {
-          long long idx = P.order ? (long long)P.order[w] : (long long)w;
-          if (!GBODE_CHECK(P, idx >= 0 && idx < P.n, CHK_ORDER)) idx = 0;
-          active = !adaptive_start<MM>(P, idx, l, tot);
-        } else {
-          exhausted = true;
-        }
-      }
-    }
-    if (!__any_sync(FULL, active)) {
-      if (!__any_sync(FULL, !exhausted)) break;
-      continue;
-    }
+    if (!feed.next<MM>(P, l, active, tot)) break;
+    if (!__any_sync(FULL, active)) continue;
     R nh[D], nc[D];
     Accepted<T> st;
     int r = TRY_REJECTED, njobs = 0;
@@ -2384,30 +2603,12 @@ __device__ __forceinline__ void run_adaptive_staged2(const KParams& P) {
 
   Lane<PR, D, F, NK> l;
   Totals tot = {0, 0, 0};
-  bool active = false, exhausted = false;
+  bool active = false;
+  Feed feed;
+  feed.init(P);
   for (;;) {
-    const bool want = !active && !exhausted;
-    const unsigned need = __ballot_sync(FULL, want);
-    if (need) {
-      const int leader = __ffs(need) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(P.counter, (unsigned long long)__popc(need));
-      base = __shfl_sync(FULL, base, leader);
-      if (want) {
-        const unsigned long long w = base + (unsigned long long)__popc(need & ((1u << lane) - 1u));
-        if (w < (unsigned long long)P.n) {
-          long long idx = P.order ? (long long)P.order[w] : (long long)w;
-          if (!GBODE_CHECK(P, idx >= 0 && idx < P.n, CHK_ORDER)) idx = 0;
-          active = !adaptive_start<M>(P, idx, l, tot);
-        } else {
-          exhausted = true;
-        }
-      }
-    }
-    if (!__any_sync(FULL, active)) {
-      if (!__any_sync(FULL, !exhausted)) break;
-      continue;
-    }
+    if (!feed.next<M>(P, l, active, tot)) break;
+    if (!__any_sync(FULL, active)) continue;
     R nh[D], nc[D];
     Accepted<T> st;
     int r = TRY_REJECTED, njobs = 0;

@@ -110,7 +110,7 @@ def test_special_stages_are_left_undecided(lib, value):
 
 
 def big_enough(pkg):
-    """An odd ensemble size just past where the integer-pipe kernels are chosen."""
+    """An odd ensemble size just past where the integer-pipe kernels are chosen (crowded() in ode_capi.cu)."""
     import torch
     return torch.cuda.get_device_properties(0).multi_processor_count * 256 + 37
 
