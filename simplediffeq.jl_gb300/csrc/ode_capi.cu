@@ -623,6 +623,24 @@ int plain_block(int64_t n, int nsm, int maxb) {
   return best;
 }
 
+/* Most blocks a persistent launch in FP64 should take for the SM
+ * sub-partitions to hold the same number of warps.  For a few more warps than
+ * there are sub-partitions some hold two, which share the FP64 pipe and end
+ * last, while the others wait; with one warp on each the lanes that finish
+ * first take the remaining trajectories.  Up to 1.4 warps a sub-partition
+ * (27,238 trajectories); above, two warps hide more latency than that costs.
+ * Time with a warp per 32 trajectories over the time so, Lorenz final states,
+ * Lotka-Volterra with saveat, linear of dimension 4 with saveat, AVern7 Van der
+ * Pol with saveat, AVern9 three-body: 20,000 trajectories 1.41, 1.16, 1.19,
+ * 1.10, 1.25; 25,000 (the first three) 1.26, 1.05, 1.16; 32,000 1.06, 0.95,
+ * 1.05, 1.02, 1.13; 38,900 (the first three) 0.92, 0.84, 0.95.  Single
+ * precision gains nothing from it. */
+int64_t even_blocks(const ode_handle* h, const ode_solve_args* a, int block) {
+  const int64_t warps = (a->n + 31) / 32, slots = (int64_t)h->nsm * 4;
+  if (a->precision != ODE_FP64 || warps <= slots || warps * 10 > slots * 14 || block > 128) return INT64_MAX;
+  return slots / (block / 32);
+}
+
 int launch(ode_handle* h, CUfunction fn, unsigned grid, int block, KParams* kp, cudaStream_t s) {
   void* params[] = {kp};
   CUresult r = g_drv.cuLaunchKernel(fn, grid, 1, 1, (unsigned)block, 1, 1, 0, (CUstream)s, params, nullptr);
@@ -1087,7 +1105,7 @@ int solve_impl(ode_handle* h, const ode_solve_args* a, ode_solve_out* o, ode_sol
     CUresult cr = g_drv.cuOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, block, 0);
     if (cr != CUDA_SUCCESS) return cu_fail(h, cr, "occupancy");
     if (nb < 1) nb = 1;
-    const int64_t resident = (int64_t)nb * h->nsm;
+    const int64_t resident = std::min<int64_t>((int64_t)nb * h->nsm, even_blocks(h, a, block));
     gridx = (unsigned)std::max<int64_t>(1, std::min<int64_t>(resident, (n + block - 1) / block));
   }
 

@@ -61,3 +61,20 @@ def test_every_step_output(pkg):
                       save_everystep=True) for s in ("plain", "persistent")]
     assert np.array_equal(a.offsets, b.offsets)
     assert np.array_equal(a.ts_rows, b.ts_rows) and np.array_equal(a.us_rows, b.us_rows)
+
+
+@pytest.mark.parametrize("nsave", [0, 5])
+@pytest.mark.parametrize("warps", [1.0, 1.001, 1.2, 1.4, 1.41, 2.0, 2.01])
+def test_sizes_around_the_launch_rules(pkg, warps, nsave):
+    """Ensembles of a given number of warps per SM sub-partition: where the persistent launch takes fewer warps than
+    the trajectories fill, and where the crowded kernels begin."""
+    import torch
+    n = int(torch.cuda.get_device_properties(0).multi_processor_count * 128 * warps)
+    u0, p = inputs("vanderpol", n, np.random.default_rng(9))
+    sv = np.linspace(0, 2.0, nsave) if nsave else None
+    ep = pkg.EnsembleProblem(pkg.ODEProblem("vanderpol", u0[:, 0], (0.0, 2.0), p[:, 0]), u0s=u0, ps=p)
+    a, b = [pkg.solve(ep, pkg.GPUSimpleATsit5(), trajectories=n, dt=0.1, abstol=1e-8, reltol=1e-6, saveat=sv, schedule=s)
+            for s in ("plain", "persistent")]
+    assert np.array_equal(a.u_final, b.u_final) and np.array_equal(a.naccept, b.naccept)
+    if nsave:
+        assert np.array_equal(a.us, b.us)
