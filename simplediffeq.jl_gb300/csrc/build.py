@@ -68,6 +68,9 @@ GROUPS = {
     "lorenz_crowded": [("atsit5", "plain", "lorenz", 3, "fp64"),
                   ("atsit5", "persistent", "lorenz", 3, "fp64")],
     "lorenz_staged_crowded": [("atsit5", "staged", "lorenz", 3, "fp64")],
+    "vdp_crowded": [("avern7", "plain", "vanderpol", 2, "fp64"),
+                    ("avern7", "persistent", "vanderpol", 2, "fp64")],
+    "vdp_staged_crowded": [("avern7", "staged", "vanderpol", 2, "fp64")],
     "kuramoto_crowded": [("atsit5", "plain", "kuramoto", 12, "fp64"),
                          ("atsit5", "persistent", "kuramoto", 12, "fp64")],
     "kuramoto_staged_crowded": [("atsit5", "staged", "kuramoto", 12, "fp64")],
@@ -85,7 +88,8 @@ GROUPS = {
 # solve: 104.8 ms with 8 warps per SM, 92.5 with 10, 84.6 with 12, 80.5 with 14,
 # 77.1 with 16).
 SHAPES = {"lorenz_staged": (64, 24576), "vdp_staged": (64, 24576), "kuramoto_staged": (32, 26112),
-          "lorenz_staged_crowded": (64, 8704), "kuramoto_staged_crowded": (32, 26112)}
+          "lorenz_staged_crowded": (64, 8704), "kuramoto_staged_crowded": (32, 26112),
+          "vdp_staged_crowded": (64, 11008)}
 
 
 def kname(alg, kind, rhs, dim, prec, crowded=False):

@@ -40,18 +40,19 @@ typedef unsigned long long ic_u64;
 /* A coefficient c of a row as the chain uses it: |c| as a 53-bit integer moved
  * up by 7 bits less the distance of its exponent from the row's largest
  * (emax, biased), so that the row's products share one scale; what is left of
- * a distance beyond 7 bits is a right shift of the product.  neg is c's sign bit. */
+ * a distance beyond 7 bits is a right shift of the product.  neg_k is c's sign
+ * bit and, below it, the stage that c multiplies. */
 struct IcTerm {
   ic_u32 a1, a0;
   ic_u32 shift;
-  ic_u32 neg;
+  ic_u32 neg_k;
 };
 IC_CX ic_u64 ic_bits(double x) { return __builtin_bit_cast(ic_u64, x); }
 IC_CX int ic_exp(double x) { return (int)(ic_bits(x) >> 52) & 0x7ff; }
-IC_CX IcTerm ic_make_term(double c, int emax) {
+IC_CX IcTerm ic_make_term(double c, int k, int emax) {
   const int dist = emax - ic_exp(c), up = dist < 7 ? 7 - dist : 0;
   const ic_u64 m = ((ic_bits(c) & 0xfffffffffffffULL) | 0x10000000000000ULL) << up;
-  return {(ic_u32)(m >> 32), (ic_u32)m, (ic_u32)(dist < 7 ? 0 : dist - 7), (ic_bits(c) >> 63) ? 0x80000000u : 0u};
+  return {(ic_u32)(m >> 32), (ic_u32)m, (ic_u32)(dist < 7 ? 0 : dist - 7), ((ic_bits(c) >> 63) ? 0x80000000u : 0u) | (ic_u32)k};
 }
 
 #if defined(__CUDACC__) || defined(__CUDACC_RTC__)
@@ -125,7 +126,7 @@ struct IcProduct {
 };
 IC_FN IcProduct ic_product(const IcTerm& c, double k, const IcSpan& E) {
   const ic_u32 kh = ic_hi(k), b0 = ic_lo(k), b1 = (kh & 0xfffffu) | 0x100000u;
-  const ic_u32 m = (ic_u32)((int)(kh ^ c.neg) >> 31), sg = m | 1u;
+  const ic_u32 m = (ic_u32)((int)(kh ^ c.neg_k) >> 31), sg = m | 1u;
   const ic_u32 d = ((E.top - 2u * kh) >> 21) + c.shift;
   const ic_u64 t = (ic_u64)c.a1 * b0 + ((ic_u64)c.a0 * b1 + ic_mulhi(c.a0, b0));
   const ic_u64 w = (ic_u64)c.a1 * b1 + (t >> 32);

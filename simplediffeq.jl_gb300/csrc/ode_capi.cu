@@ -300,9 +300,9 @@ int kernel_kind_id(const char* k) {
 /* Bytes of one saveat job in the staged kernel's ring: the host-side copy of
  * StageLayout<M, PR, D, F>::JOB in ode_solver.cuh (3 times of type T, the
  * trajectory index, the saveat index, and D (x2 with Kahan) state values,
- * NK x D stage values and, for the Verner methods, the parameters, of type R). */
+ * DK x D stage values and, for the Verner methods, the parameters, of type R). */
 int stage_job_bytes(const ode_solve_args* a) {
-  const int nk = a->alg == ODE_ALG_AVERN9 ? 16 : a->alg == ODE_ALG_AVERN7 ? 10 : 7;
+  const int nk = a->alg == ODE_ALG_AVERN9 ? 9 : 7;  /* the methods' DK */
   const int r = a->precision == ODE_FP64 ? 8 : 4, t = a->precision == ODE_FP32 ? 4 : 8;
   const bool dense_f = a->alg != ODE_ALG_ATSIT5;  /* Verner dense output evaluates f: parameters ride along */
   const int nrec = a->dim * (a->precision == ODE_FP32_KAHAN ? 2 : 1) + nk * a->dim + (dense_f ? a->nparams : 0);
@@ -317,7 +317,7 @@ int stage_job_bytes(const ode_solve_args* a) {
 int stage_record_bytes(const ode_solve_args* a) {
   const int nx = a->alg == ODE_ALG_AVERN9 ? 10 : a->alg == ODE_ALG_AVERN7 ? 6 : 0;
   if (!nx) return 0;
-  const int nk = a->alg == ODE_ALG_AVERN9 ? 16 : 10;
+  const int nk = a->alg == ODE_ALG_AVERN9 ? 9 : 7;
   const int r = a->precision == ODE_FP64 ? 8 : 4, t = a->precision == ODE_FP32 ? 4 : 8;
   const int nrec = a->dim * (a->precision == ODE_FP32_KAHAN ? 2 : 1) + nk * a->dim + a->nparams + nx * a->dim;
   return 3 * t + 8 + 4 + nrec * r + 2 * 8;
@@ -332,22 +332,30 @@ int stage_unit_bytes(const ode_solve_args* a) {
 
 /* Bytes of shared memory a warp of the integer-pipe kernels keeps its stages
  * in: the host-side copy of Stages<...>::BYTES in ode_solver.cuh. */
-int stage_slice_bytes(const ode_solve_args* a) { return 7 * a->dim * 32 * 8; }
+int stage_slice_bytes(const ode_solve_args* a) { return (a->alg == ODE_ALG_AVERN7 ? 10 : 7) * a->dim * 32 * 8; }
 
 /* A ring of 36 units, in steps of 512 bytes: a round of 32 and a few more. */
 int small_ring_bytes(const ode_solve_args* a) { return (36 * stage_unit_bytes(a) + 511) / 512 * 512; }
 
 /* Whether the ensemble crowds the GPU: more than two warps of trajectories for
- * every SM sub-partition (38,912).  Adaptive Tsit5 in FP64 and the default
- * rounding has kernels of its own for that (GBODE_CROWDED): their warps merge
- * when the ensemble runs out (Feed), and where they fit they run linear
- * combinations on the integer pipe.  The smaller ensembles' kernels do
+ * every SM sub-partition (38,912).  Adaptive Tsit5 and Verner 7 in FP64 and the
+ * default rounding have kernels of their own for that (GBODE_CROWDED): their
+ * warps merge when the ensemble runs out (Feed), and where they fit they run
+ * linear combinations on the integer pipe.  The smaller ensembles' kernels do
  * without the code for it, whose few instructions an attempt cost a lone
- * trajectory 0.6%. */
+ * trajectory 0.6%.
+ *
+ * Verner 7 with saveat: five warps.  Its step records leave shared memory for
+ * fewer warps, which the integer pipe's latency needs; time of the register
+ * kernel over the crowded one's on Van der Pol, 0 / 20 / 200 save points:
+ * 50,000 trajectories 1.32 / 1.06 / 0.95, 100,000 1.26 / 1.07 / 1.02, 200,003
+ * 1.23 / 1.10 / 1.05.  Verner 9 on the three-body problem: 0.95 to 1.05. */
 bool crowded(const ode_handle* h, const ode_solve_args* a) {
-  if (a->alg != ODE_ALG_ATSIT5 || a->precision != ODE_FP64 || a->controller == ODE_CTRL_REF) return false;
+  if ((a->alg != ODE_ALG_ATSIT5 && a->alg != ODE_ALG_AVERN7) || a->precision != ODE_FP64 ||
+      a->controller == ODE_CTRL_REF)
+    return false;
   if (h->tune_crowded >= 0) return h->tune_crowded != 0;
-  return a->n > (int64_t)h->nsm * 4 * 64;
+  return a->n > (int64_t)h->nsm * 4 * (a->alg == ODE_ALG_AVERN7 && a->nsave > 0 ? 160 : 64);
 }
 
 /* Whether its kernel keeps the stages in shared memory and forms their linear
@@ -390,7 +398,7 @@ void default_shape(const ode_handle* h, const ode_solve_args* a, int sched, int*
   }
   if (!staged) return;
   const int unit = stage_unit_bytes(a);
-  if (((12288 / unit) & ~7) >= 32) return;
+  if (12288 / unit >= 32) return;
   const int fit = (32 * unit + 511) / 512 * 512;
   if (fit > 49152) return;  /* no ring holds a round: the kernel runs unstaged */
   *block = 32;
@@ -1712,7 +1720,7 @@ int ode_autotune(ode_handle* h, const ode_solve_args* a, int64_t sample, ode_tun
     if (staged) {
       if ((ic || fit > 12288) && fit / 32 * block <= 49152) rings.push_back(fit);
       for (int ring : {12288, 16384, 24576, 36864, 49152})
-        if (ring / 32 * block <= 49152 && (ring / job & ~7) >= 32) rings.push_back(ring);
+        if (ring / 32 * block <= 49152 && ring / job >= 32) rings.push_back(ring);
     }
     if (rings.empty()) rings.push_back(12288);
     for (int regs : {0, 128, 112, 96, 80})

@@ -838,12 +838,14 @@ struct RhsLinear {
 
 /* ------------------------------------------------------------------ Tsitouras 5(4) */
 /* src/tsit5/gpuatsit5.jl:258-275 (stages, FSAL k7), :306-314 and
- * src/tsit5/tsit5.jl:385-399 (dense output). */
+ * src/tsit5/tsit5.jl:385-399 (dense output).
+ * Every method: NK stages; DK of them enter the dense output (and wait for it
+ * in the staging rings), the first and those from 1 + DSKIP on. */
 template <class PR, int D, class F>
 struct MTsit5 {
   typedef typename PR::R R;
   typedef typename PR::T T;
-  enum { NK = 7, FSAL = 1, DTMIN_1F7 = 0, DENSE_F = 0, NX = 0, IC = 1 };  /* DENSE_F: dense output evaluates f */
+  enum { NK = 7, FSAL = 1, DTMIN_1F7 = 0, DENSE_F = 0, NX = 0, DK = 7, DSKIP = 0 };  /* DENSE_F: dense output evaluates f */
 
   __device__ static __forceinline__ void attempt(const F& f, const R (&uh)[D], const R (&uc)[D], T t, T dt,
                                                  R (&k)[NK][D], R (&nh)[D], R (&nc)[D], R (&e)[D], bool want_err) {
@@ -911,7 +913,7 @@ template <class PR, int D, class F>
 struct MVern7 {
   typedef typename PR::R R;
   typedef typename PR::T T;
-  enum { NK = 10, FSAL = 0, DTMIN_1F7 = 0, DENSE_F = 1, IC = 0 };
+  enum { NK = 10, FSAL = 0, DTMIN_1F7 = 0, DENSE_F = 1, DK = 7, DSKIP = 2 };
 
   __device__ static __forceinline__ void attempt(const F& f, const R (&uh)[D], const R (&uc)[D], T t, T dt,
                                                  R (&k)[NK][D], R (&nh)[D], R (&nc)[D], R (&e)[D], bool want_err) {
@@ -1033,7 +1035,7 @@ template <class PR, int D, class F, bool ADAPTIVE>
 struct MVern9Impl {
   typedef typename PR::R R;
   typedef typename PR::T T;
-  enum { NK = 16, FSAL = 0, DTMIN_1F7 = 1, DENSE_F = 1, IC = 0 };
+  enum { NK = 16, FSAL = 0, DTMIN_1F7 = 1, DENSE_F = 1, DK = 9, DSKIP = ADAPTIVE ? 6 : 0 };
 
   __device__ static __forceinline__ void attempt(const F& f, const R (&uh)[D], const R (&uc)[D], T t, T dt,
                                                  R (&k)[NK][D], R (&nh)[D], R (&nc)[D], R (&e)[D], bool want_err) {
@@ -1300,12 +1302,31 @@ struct StageRows {
   __device__ __forceinline__ StageRow<R, STRIDE> operator[](int q) const { return StageRow<R, STRIDE>{p + q * D * STRIDE}; }
 };
 
-static_assert(tsit5_btilde7 == tsit5_btilde1 + 6, "the error weights are consecutive");
+/* What the integer-pipe attempt of a method walks: its rows and those of its
+ * extra dense-output stages, and the weights of the error estimate and the
+ * stages they multiply. */
+template <class M> struct IcMethod { enum { HAS = 0 }; };
+template <class PR, int D, class F> struct IcMethod<MTsit5<PR, D, F>> {
+  typedef IcT5 Rows;
+  typedef IcT5 Extra; /* none */
+  enum { HAS = 1, NE = 7 };
+  __device__ static __forceinline__ int estage(int j) { return j; }
+  __device__ static __forceinline__ double ecoef(int j) { return c_tsit5_d[tsit5_btilde1 + j]; }
+};
+template <class PR, int D, class F> struct IcMethod<MVern7<PR, D, F>> {
+  typedef IcV7 Rows;
+  typedef IcV7X Extra;
+  enum { HAS = 1, NE = 8 };
+  __device__ static __forceinline__ int estage(int j) { return j == 0 ? 0 : j + 2; }
+  __device__ static __forceinline__ double ecoef(int j) { return c_vern7_d[vern7_btilde1 + j]; }
+};
+static_assert(tsit5_btilde7 == tsit5_btilde1 + 6 && vern7_btilde10 == vern7_btilde1 + 7 &&
+              vern7_btilde4 == vern7_btilde1 + 1, "the error weights are consecutive");
 
-/* Tsit5's attempt with the stages in shared memory and their linear
+/* A method's attempt with the stages in shared memory and their linear
  * combinations on the integer pipe (intchain.h): the same values as
- * MTsit5::attempt.  The FP64 pipe bounds the solve; of an attempt's 162 FP64
- * instructions on Lorenz this leaves 99: the right-hand sides, the state
+ * M::attempt.  The FP64 pipe bounds the solve; of an attempt's 162 FP64
+ * instructions with Tsit5 on Lorenz this leaves 99: the right-hand sides, the state
  * updates u + h s (whose two terms can be 2^40 apart) and the error estimate
  * (whose sum cancels 20 bits and more: undecided in 8 rows of 10).
  *
@@ -1319,31 +1340,40 @@ template <class M, class PR, int D, class F>
 struct MInt : M {
   typedef typename PR::R R;
   typedef typename PR::T T;
+  typedef IcMethod<M> IM;
+  typedef typename IM::Rows Rows;
+  typedef typename IM::Extra Extra;
 
-  /* s = sum_j c_j k_j of a row, whose term j multiplies stage j, by fused
-   * multiply-adds as lc() does it */
-  template <int STRIDE>
+  /* the stage that term j of a row multiplies: stage j where the table says so;
+   * a staged step's extra stages, from DK on, lie GAP values further */
+  template <class TAB, int STRIDE, int GAP>
+  __device__ static __forceinline__ const R* stage_of(const IcTerm& c, int j, const R* kb) {
+    const int k = TAB::CONSECUTIVE ? j : (int)(c.neg_k & 0xffu);
+    return kb + (k * D + (GAP && k >= M::DK ? GAP : 0)) * STRIDE;
+  }
+  /* s = sum_j c_j k_j of a row by fused multiply-adds as lc() does it */
+  template <class TAB, int STRIDE, int GAP>
   __device__ static __forceinline__ void row_fma(const IcRow& row, const R* kb, R (&s)[D]) {
 #pragma unroll
-    for (int d = 0; d < D; ++d) s[d] = c_ic_t5.coef[row.first] * kb[d * STRIDE];
+    for (int d = 0; d < D; ++d) s[d] = TAB::coef(row.first) * kb[d * STRIDE];
 #pragma unroll 1
     for (int j = 1; j < row.n; ++j) {
-      const R c = c_ic_t5.coef[row.first + j];
-      const R* kp = kb + j * D * STRIDE;
+      const R c = TAB::coef(row.first + j);
+      const R* kp = stage_of<TAB, STRIDE, GAP>(TAB::term(row.first + j), j, kb);
 #pragma unroll
       for (int d = 0; d < D; ++d) s[d] = fmaR(c, kp[d * STRIDE], s[d]);
     }
   }
   /* the same on the integer pipe; false if a component's sum was not decided there */
-  template <int STRIDE>
+  template <class TAB, int STRIDE, int GAP>
   __device__ static __forceinline__ bool row_int(const IcRow& row, const R* kb, const IcSpan (&E)[D], R (&s)[D]) {
     IcSum S[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) S[d] = IcSum{0u, 0u, 0u, false};
 #pragma unroll 1
     for (int j = 0; j < row.n; ++j) {
-      const IcTerm c = c_ic_t5.term[row.first + j];
-      const R* kp = kb + j * D * STRIDE;
+      const IcTerm c = TAB::term(row.first + j);
+      const R* kp = stage_of<TAB, STRIDE, GAP>(c, j, kb);
 #pragma unroll
       for (int d = 0; d < D; ++d) ic_add_product(S[d], ic_product(c, kp[d * STRIDE], E[d]));
     }
@@ -1356,12 +1386,12 @@ struct MInt : M {
     return ok;
   }
   /* whichever applies; false if the integer pipe was tried and left the row undecided */
-  template <int STRIDE>
+  template <class TAB, int STRIDE, int GAP>
   __device__ static __forceinline__ bool row_sum(const IcRow& row, const R* kb, const IcSpan (&E)[D], bool on_int,
                                                  R (&s)[D]) {
     bool done = false;
-    if (on_int) done = row_int<STRIDE>(row, kb, E, s);
-    if (!done) row_fma<STRIDE>(row, kb, s);
+    if (on_int) done = row_int<TAB, STRIDE, GAP>(row, kb, E, s);
+    if (!done) row_fma<TAB, STRIDE, GAP>(row, kb, s);
     return done || !on_int;
   }
 
@@ -1377,24 +1407,30 @@ struct MInt : M {
     bool missed = false;
     R tmp[D], du[D];
     IcSpan E[D];
+    if (!M::FSAL) {
+      f(uh, t, du);
+#pragma unroll
+      for (int d = 0; d < D; ++d) k[0][d] = du[d];
+    }
 #pragma unroll
     for (int d = 0; d < D; ++d) E[d] = ic_span(k[0][d]);
 #pragma unroll 1
-    for (int r = 0; r < kRowsT5; ++r) {
-      const IcRow row = c_ic_t5.row[r];
+    for (int r = 0; r < Rows::NR; ++r) {
+      const IcRow row = Rows::row(r);
       if (r == 0) {
-        const R a = (R)(dt * c_ic_t5.coef[0]);
+        const R a = (R)(dt * Rows::coef(0));
 #pragma unroll
         for (int d = 0; d < D; ++d) tmp[d] = fmaR(a, k[0][d], uh[d]);
       } else {
         R s[D];
-        missed = !row_sum<STRIDE>(row, k.p, E, on_int, s) || missed;
+        missed = !row_sum<Rows, STRIDE, 0>(row, k.p, E, on_int, s) || missed;
         axpy(tmp, uh, h, s);
       }
+      if (!M::FSAL && row.out < 0) break;
       f(tmp, stime(t, row.c, dt), du);
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        k.p[((r + 1) * D + d) * STRIDE] = du[d];
+        k.p[(row.out * D + d) * STRIDE] = du[d];
         ic_widen(E[d], du[d]);
       }
     }
@@ -1404,18 +1440,47 @@ struct MInt : M {
     for (int d = 0; d < D; ++d) {
       nh[d] = tmp[d];
       nc[d] = (R)0;
-      e[d] = c_tsit5_d[tsit5_btilde1] * k[0][d];
+      e[d] = IM::ecoef(0) * k[0][d];
     }
 #pragma unroll 1
-    for (int j = 1; j < M::NK; ++j) {
-      const R c = c_tsit5_d[tsit5_btilde1 + j];
-      const R* kp = k.p + j * D * STRIDE;
+    for (int j = 1; j < IM::NE; ++j) {
+      const R c = IM::ecoef(j);
+      const R* kp = k.p + IM::estage(j) * D * STRIDE;
 #pragma unroll
       for (int d = 0; d < D; ++d) e[d] = fmaR(c, kp[d * STRIDE], e[d]);
     }
     if (!ErrUnscaled<R>::value) {
 #pragma unroll
       for (int d = 0; d < D; ++d) e[d] = h * e[d];
+    }
+  }
+
+  /* The extra dense-output stages of the staged step whose DK stages lie at kb,
+   * written GAP values after them: the values of M::dense_stages. */
+  template <int STRIDE, int GAP>
+  __device__ static __forceinline__ void dense_stages_at(const F& f, const R (&uh)[D], T tnew, T dtold, R* kb) {
+    const R h = (R)dtold;
+    IcSpan E[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) E[d] = ic_span(kb[d * STRIDE]);
+#pragma unroll 1
+    for (int j = 1; j < Extra::row(0).n; ++j) {
+      const R* kp = stage_of<Extra, STRIDE, GAP>(Extra::term(j), j, kb);
+#pragma unroll
+      for (int d = 0; d < D; ++d) ic_widen(E[d], kp[d * STRIDE]);
+    }
+#pragma unroll 1
+    for (int r = 0; r < Extra::NR; ++r) {
+      const IcRow row = Extra::row(r);
+      R s[D], tmp[D], du[D];
+      row_sum<Extra, STRIDE, GAP>(row, kb, E, true, s);
+      axpy(tmp, uh, h, s);
+      f(tmp, stime(tnew, row.c, dtold), du);
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        kb[(row.out * D + GAP + d) * STRIDE] = du[d];
+        ic_widen(E[d], du[d]);
+      }
     }
   }
 };
@@ -1433,7 +1498,7 @@ enum { CROWDED = 0 };
 template <class M, class PR, int D, class F, int RING>
 struct Stages {
   enum { BYTES = M::NK * D * 32 * 8 };
-  enum { SHARED = CROWDED && M::IC && sizeof(typename PR::R) == 8 && BYTES + RING <= 19456 &&
+  enum { SHARED = CROWDED && IcMethod<M>::HAS && sizeof(typename PR::R) == 8 && BYTES + RING <= 19456 &&
                   (GBODE_BLOCK / 32) * (BYTES + RING) <= 49152 };
 };
 template <bool SHARED, class M, class PR, int D, class F> struct StageTypes {
@@ -2333,9 +2398,9 @@ struct StageLayout {
   typedef typename PR::R R;
   typedef typename PR::T T;
   /* the parameters ride along only when the dense output evaluates f (Verner's extra stages) */
-  enum { NREC = D * (PR::KAHAN ? 2 : 1) + M::NK * D + (M::DENSE_F ? F::NP : 0) };
+  enum { NREC = D * (PR::KAHAN ? 2 : 1) + M::DK * D + (M::DENSE_F ? F::NP : 0) };
   enum { JOB = 3 * (int)sizeof(T) + 8 + NREC * (int)sizeof(R) + 4 };
-  enum { CAP = (kStageBytesPerWarp / JOB) & ~7 };
+  enum { CAP = (kStageBytesPerWarp / JOB) & ~1 };
 };
 
 /* The stage values of one staged job as the dense formulas index them,
@@ -2349,11 +2414,11 @@ struct RingRow {
   const R* p;
   __device__ __forceinline__ R operator[](int d) const { return p[d * STRIDE]; }
 };
-template <class R, int D, int STRIDE>
+template <class R, int D, int STRIDE, int SKIP>
 struct RingStages {
   const R* p;
   __device__ __forceinline__ RingRow<R, STRIDE> operator[](int q) const {
-    return RingRow<R, STRIDE>{p + q * D * STRIDE};
+    return RingRow<R, STRIDE>{p + (q == 0 ? 0 : q - SKIP) * D * STRIDE};
   }
 };
 
@@ -2362,7 +2427,7 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P, typename P
   typedef typename PR::R R;
   typedef typename PR::T T;
   typedef StageLayout<M, PR, D, F> SL;
-  enum { CAP = SL::CAP, NK = M::NK, KOFF = D * (PR::KAHAN ? 2 : 1), POFF = KOFF + NK * D };
+  enum { CAP = SL::CAP, NK = M::NK, DK = M::DK, KOFF = D * (PR::KAHAN ? 2 : 1), POFF = KOFF + DK * D };
   __shared__ __align__(16) unsigned char qmem[kWarpsPerBlock][kStageBytesPerWarp];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -2394,7 +2459,7 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P, typename P
         uh[d] = rv[d * CAP + slot];
         uc[d] = PR::KAHAN ? rv[(D + d) * CAP + slot] : (R)0;
       }
-      const RingStages<R, D, CAP> kk{rv + KOFF * CAP + slot};
+      const RingStages<R, D, CAP, M::DSKIP> kk{rv + KOFF * CAP + slot};
       if (M::DENSE_F) {
 #pragma unroll
         for (int q = 0; q < F::NP; ++q) f2.p[q] = rv[(POFF + q) * CAP + slot];
@@ -2457,9 +2522,9 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P, typename P
             if (PR::KAHAN) rv[(D + d) * CAP + slot] = l.uc[d];
           }
 #pragma unroll
-          for (int k = 0; k < NK; ++k)
+          for (int k = 0; k < DK; ++k)
 #pragma unroll
-            for (int d = 0; d < D; ++d) rv[(KOFF + k * D + d) * CAP + slot] = l.k[k][d];
+            for (int d = 0; d < D; ++d) rv[(KOFF + k * D + d) * CAP + slot] = l.k[k == 0 ? 0 : k + M::DSKIP][d];
           if (M::DENSE_F) {
 #pragma unroll
             for (int k = 0; k < F::NP; ++k) rv[(POFF + k) * CAP + slot] = l.f.p[k];
@@ -2506,19 +2571,19 @@ template <class M, class PR, int D, class F>
 struct StageLayout2 {
   typedef typename PR::R R;
   typedef typename PR::T T;
-  enum { KOFF = D * (PR::KAHAN ? 2 : 1), POFF = KOFF + M::NK * D, XOFF = POFF + F::NP, NREC = XOFF + M::NX * D };
+  enum { KOFF = D * (PR::KAHAN ? 2 : 1), POFF = KOFF + M::DK * D, XOFF = POFF + F::NP, NREC = XOFF + M::NX * D };
   /* bytes of a record (3 times, trajectory, point count, values) and of a point (record slot, saveat index) */
   enum { REC = 3 * (int)sizeof(T) + 8 + 4 + NREC * (int)sizeof(R), PT = 8 };
   /* room for twice as many points as records */
-  enum { CR = (kStageBytesPerWarp / (REC + 2 * PT)) & ~7, CP = 2 * CR };
+  enum { CR = (kStageBytesPerWarp / (REC + 2 * PT)) & ~1, CP = 2 * CR };
 };
 
 template <class M, class PR, int D, class F>
-__device__ __forceinline__ void run_adaptive_staged2(const KParams& P) {
+__device__ __forceinline__ void run_adaptive_staged2(const KParams& P, typename PR::R* slice) {
   typedef typename PR::R R;
   typedef typename PR::T T;
   typedef StageLayout2<M, PR, D, F> SL;
-  enum { CR = SL::CR, CP = SL::CP, NK = M::NK, NX = M::NX, KOFF = SL::KOFF, POFF = SL::POFF, XOFF = SL::XOFF,
+  enum { CR = SL::CR, CP = SL::CP, NK = M::NK, DK = M::DK, NX = M::NX, KOFF = SL::KOFF, POFF = SL::POFF, XOFF = SL::XOFF,
          NREC = SL::NREC };
   __shared__ __align__(16) unsigned char qmem[kWarpsPerBlock][kStageBytesPerWarp];
   const unsigned FULL = 0xffffffffu;
@@ -2549,13 +2614,18 @@ __device__ __forceinline__ void run_adaptive_staged2(const KParams& P) {
       }
 #pragma unroll
       for (int q = 0; q < F::NP; ++q) f2.p[q] = rv[(POFF + q) * CR + slot];
-      const RingStages<R, D, CR> kk{rv + KOFF * CR + slot};
-      R x[NX][D];
-      M::dense_stages(f2, uh, uc, tv[slot], tv[CR + slot], tv[2 * CR + slot], kk, x);
+      if constexpr (Stages<M, PR, D, F, kStageBytesPerWarp>::SHARED) {
+        MInt<M, PR, D, F>::template dense_stages_at<CR, XOFF - POFF>(f2, uh, tv[CR + slot], tv[2 * CR + slot],
+                                                                     rv + KOFF * CR + slot);
+      } else {
+        const RingStages<R, D, CR, M::DSKIP> kk{rv + KOFF * CR + slot};
+        R x[NX][D];
+        M::dense_stages(f2, uh, uc, tv[slot], tv[CR + slot], tv[2 * CR + slot], kk, x);
 #pragma unroll
-      for (int q = 0; q < NX; ++q)
+        for (int q = 0; q < NX; ++q)
 #pragma unroll
-        for (int d = 0; d < D; ++d) rv[(XOFF + q * D + d) * CR + slot] = x[q][d];
+          for (int d = 0; d < D; ++d) rv[(XOFF + q * D + d) * CR + slot] = x[q][d];
+      }
       np = nv[slot];
     }
 #pragma unroll
@@ -2581,8 +2651,8 @@ __device__ __forceinline__ void run_adaptive_staged2(const KParams& P) {
       }
       const T told = tv[slot], dtold = tv[2 * CR + slot];
       const T theta = theta_of((T)P.saveat[j], told, dtold, recip(dtold));
-      const RingStages<R, D, CR> kk{rv + KOFF * CR + slot};
-      const RingStages<R, D, CR> xx{rv + XOFF * CR + slot};
+      const RingStages<R, D, CR, M::DSKIP> kk{rv + KOFF * CR + slot};
+      const RingStages<R, D, CR, 0> xx{rv + XOFF * CR + slot};
       double v[D];
       M::dense_eval(uh, uc, dtold, theta, kk, xx, v);
       store_point<PR, D>(P, iv[slot], j, v);
@@ -2601,19 +2671,22 @@ __device__ __forceinline__ void run_adaptive_staged2(const KParams& P) {
     }
   };
 
-  Lane<PR, D, F, NK> l;
+  typedef StageTypes<Stages<M, PR, D, F, kStageBytesPerWarp>::SHARED, M, PR, D, F> ST;
+  typedef typename ST::Method MM;
+  Lane<PR, D, F, NK, typename ST::KS> l;
+  ST::bind(l.k, slice);
   Totals tot = {0, 0, 0};
   bool active = false;
   Feed feed;
   feed.init(P);
   for (;;) {
-    if (!feed.next<M>(P, l, active, tot)) break;
+    if (!feed.next<MM>(P, l, active, tot)) break;
     if (!__any_sync(FULL, active)) continue;
     R nh[D], nc[D];
     Accepted<T> st;
     int r = TRY_REJECTED, njobs = 0;
     if (active) {
-      r = adaptive_try<M>(P, l, tot, nh, nc, st);
+      r = adaptive_try<MM>(P, l, tot, nh, nc, st);
       if (r == TRY_STOPPED) active = false;
       if (r == TRY_ACCEPTED)
         while (l.cur + njobs < P.nsave && t_le<PR>(P.saveat[l.cur + njobs], l.t)) ++njobs;
@@ -2650,9 +2723,9 @@ __device__ __forceinline__ void run_adaptive_staged2(const KParams& P) {
             if (PR::KAHAN) rv[(D + d) * CR + slot] = l.uc[d];
           }
 #pragma unroll
-          for (int k = 0; k < NK; ++k)
+          for (int k = 0; k < DK; ++k)
 #pragma unroll
-            for (int d = 0; d < D; ++d) rv[(KOFF + k * D + d) * CR + slot] = l.k[k][d];
+            for (int d = 0; d < D; ++d) rv[(KOFF + k * D + d) * CR + slot] = l.k[k == 0 ? 0 : k + M::DSKIP][d];
 #pragma unroll
           for (int k = 0; k < F::NP; ++k) rv[(POFF + k) * CR + slot] = l.f.p[k];
           for (int q = 0; q < njobs; ++q) {
@@ -2680,7 +2753,7 @@ __device__ __forceinline__ void run_adaptive_staged2(const KParams& P) {
     }
     (void)GBODE_CHECK(P, rc >= 0 && rc <= CR && pc >= 0 && pc <= CP && rs <= rc && pr <= pc, CHK_RING);
     if (r == TRY_ACCEPTED) {
-      adaptive_commit<M>(l, nh, nc);
+      adaptive_commit<MM>(l, nh, nc);
       store_step<PR, D>(P, l, l.nacc);
       if (!t_lt<PR>(l.t, P.tf)) {
         lane_finish(P, l, RET_DEFAULT, tot);
@@ -2706,7 +2779,7 @@ __device__ __forceinline__ void run_adaptive_staged_or_persistent(const KParams&
   typename PR::R* slice = kmem[threadIdx.x >> 5];
   if constexpr (two) {
     if (P.nsave > 0) {
-      run_adaptive_staged2<M, PR, D, F>(P);
+      run_adaptive_staged2<M, PR, D, F>(P, slice);
       return;
     }
   } else if constexpr (one) {
