@@ -50,6 +50,7 @@
 #include <cstdio>
 #include <cstring>
 #include <random>
+#include <utility>
 #include <vector>
 
 #include "ode_host.h"
@@ -67,7 +68,10 @@ constexpr int NBINS = kCostBins;
 constexpr int NH = 64;          /* hidden units; narrower models are zero-padded (padded units stay zero) */
 constexpr int LDH = NH + 8;     /* bf16 row stride of hidden-width tiles: 144 B, ldmatrix rows on distinct banks */
 constexpr int W3ROWS = 8;       /* output rows padded to one n8 tile */
-constexpr int TW = 8;           /* warps per training CTA */
+constexpr int TW = 8;           /* warps of a training CTA that compute on samples */
+constexpr int TT = 320;         /* its threads: with two more warps an owner slice of 16 (297 parameters for six
+                                   inputs) takes one round of remote loads and stores instead of two */
+constexpr int TU = 3;           /* rounds at most (40 inputs, 8 CTAs: 865 parameters) */
 constexpr int TROWS = 16 * TW;  /* samples per training tile */
 constexpr int PW = 8;           /* warps per prediction block */
 
@@ -434,9 +438,15 @@ __device__ __forceinline__ uint32_t permute(uint32_t i, const Perm& p) {
 }
 
 /* One thread-block cluster trains the network for every epoch (see the file
- * comment).  Grid = the cluster: CSIZE CTAs of TW warps. */
+ * comment).  Grid = the cluster: CSIZE CTAs of TT threads.
+ *
+ * A step is a chain of small dependent products between two cluster barriers,
+ * bound by latency.  What does not depend on the other CTAs (the next tile's
+ * gather, the step's Adam constants) runs between a barrier's arrive and its
+ * wait, a tile's first gradient is stored, not added to a zeroed array, and
+ * where a parameter lies is worked out once, not every step: MEASURED. */
 template <int KIN, int CSIZE>
-__global__ void __launch_bounds__(TW * 32, 1) mlp_train(TrainParams tp) {
+__global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
   constexpr int csize = CSIZE;
   extern __shared__ __align__(16) unsigned char smem[];
   cg::cluster_group cluster = cg::this_cluster();
@@ -471,9 +481,13 @@ __global__ void __launch_bounds__(TW * 32, 1) mlp_train(TrainParams tp) {
 
   /* initial network, owner slice, zeroed output-delta padding */
   load_net(net, nin, nh, [&](int i) { return tp.master[i]; });
-  for (int i = lo + tid; i < hi; i += blockDim.x) {
-    const ParamSlot s = param_slot(i, nin, nh, ldx);
-    ow[i - lo] = s.ext >= 0 ? tp.master[s.ext] : 0.f;
+  ParamSlot slot[TU]; /* this thread's parameters of the owner slice */
+#pragma unroll
+  for (int u = 0; u < TU; ++u) {
+    const int i = lo + tid + u * TT;
+    if (i >= hi) break;
+    slot[u] = param_slot(i, nin, nh, ldx);
+    ow[i - lo] = slot[u].ext >= 0 ? tp.master[slot[u].ext] : 0.f;
     om[i - lo] = 0.f;
     ov[i - lo] = 0.f;
   }
@@ -494,7 +508,8 @@ __global__ void __launch_bounds__(TW * 32, 1) mlp_train(TrainParams tp) {
     const int sie = tp.grad_only ? 0 : st % tp.steps_per_epoch;
     const Perm perm = make_perm((uint32_t)tp.nb, tp.seed_lo, tp.seed_hi,
                                 (uint32_t)(tp.grad_only ? 0 : st / tp.steps_per_epoch));
-    for (int i = tid; i < TROWS * 2; i += blockDim.x) {
+    const int rows = (valid + 15) & ~15; /* what the products read */
+    for (int i = tid; i < rows * 2; i += blockDim.x) {
       const int s = i >> 1, half = i & 1;
       int idx = -1;
       if (s < valid) {
@@ -511,7 +526,8 @@ __global__ void __launch_bounds__(TW * 32, 1) mlp_train(TrainParams tp) {
   for (int step = 0; step < total_steps; ++step) {
     const int epoch = tp.grad_only ? 0 : step / tp.steps_per_epoch;
     const int sie = tp.grad_only ? 0 : step % tp.steps_per_epoch;
-    for (int i = tid; i < L.P; i += blockDim.x) gp[i] = 0.f;
+    if (my0 >= my1)
+      for (int i = tid; i < L.P; i += blockDim.x) gp[i] = 0.f;
 
     for (int r0 = my0; r0 < my1; r0 += TROWS) {
       const int valid = min(TROWS, my1 - r0);
@@ -597,8 +613,11 @@ __global__ void __launch_bounds__(TW * 32, 1) mlp_train(TrainParams tp) {
         }
       }
       __syncthreads();
-      /* weight gradients over the tile's samples (K = samples, operands read transposed) */
-      {
+      /* weight gradients over the tile's samples (K = samples, operands read transposed); the first tile's are
+       * stored, the others' added */
+      const bool first = r0 == my0;
+      auto put = [&](int i, float v) { gp[i] = first ? v : gp[i] + v; };
+      if (warp < TW) {
         /* gW2[j][k] = sum_s d2[s][j] h1[s][k]; gb2[j] = sum_s d2[s][j] (ones operand) */
         const int mt = warp >> 1, nb0 = (warp & 1) * 32;
         float acc[4][4] = {};
@@ -621,21 +640,21 @@ __global__ void __launch_bounds__(TW * 32, 1) mlp_train(TrainParams tp) {
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
           const int j = mt * 16 + g, k = nb0 + nt * 8 + 2 * t;
-          gp[gw2 + j * NH + k] += acc[nt][0];
-          gp[gw2 + j * NH + k + 1] += acc[nt][1];
-          gp[gw2 + (j + 8) * NH + k] += acc[nt][2];
-          gp[gw2 + (j + 8) * NH + k + 1] += acc[nt][3];
+          put(gw2 + j * NH + k, acc[nt][0]);
+          put(gw2 + j * NH + k + 1, acc[nt][1]);
+          put(gw2 + (j + 8) * NH + k, acc[nt][2]);
+          put(gw2 + (j + 8) * NH + k + 1, acc[nt][3]);
         }
         if (bias && t == 0) {
-          gp[gb2 + mt * 16 + g] += accb[0];
-          gp[gb2 + mt * 16 + g + 8] += accb[2];
+          put(gb2 + mt * 16 + g, accb[0]);
+          put(gb2 + mt * 16 + g + 8, accb[2]);
         }
       }
       {
         /* gW1[j][f] = sum_s d1[s][j] x[s][f]; gb1[j] = sum_s d1[s][j] */
         const int gw1 = 0, gb1 = NH * nin;
         const uint32_t ones = g == 0 ? kOnesBf16x2 : 0u;
-        for (int id = warp; id < 8 * KIN; id += TW) {
+        for (int id = warp; id < (warp < TW ? 8 * KIN : 0); id += TW) {
           const int mt = id & 3, nt = id >> 2;
           float acc[4] = {};
           float accb[4] = {};
@@ -649,16 +668,16 @@ __global__ void __launch_bounds__(TW * 32, 1) mlp_train(TrainParams tp) {
           }
           const int j = mt * 16 + g, f = nt * 8 + 2 * t;
           if (f < nin) {
-            gp[gw1 + j * nin + f] += acc[0];
-            gp[gw1 + (j + 8) * nin + f] += acc[2];
+            put(gw1 + j * nin + f, acc[0]);
+            put(gw1 + (j + 8) * nin + f, acc[2]);
           }
           if (f + 1 < nin) {
-            gp[gw1 + j * nin + f + 1] += acc[1];
-            gp[gw1 + (j + 8) * nin + f + 1] += acc[3];
+            put(gw1 + j * nin + f + 1, acc[1]);
+            put(gw1 + (j + 8) * nin + f + 1, acc[3]);
           }
           if (bias && t == 0) {
-            gp[gb1 + mt * 16 + g] += accb[0];
-            gp[gb1 + mt * 16 + g + 8] += accb[2];
+            put(gb1 + mt * 16 + g, accb[0]);
+            put(gb1 + mt * 16 + g + 8, accb[2]);
           }
         }
       }
@@ -678,36 +697,40 @@ __global__ void __launch_bounds__(TW * 32, 1) mlp_train(TrainParams tp) {
         const int gw3 = NH * nin + 2 * NH + NH * NH, gb3 = gw3 + NOUT * NH;
         if (t == 0) {
           const int k = mt * 16 + g;
-          gp[gw3 + k] += acc[0];
-          gp[gw3 + NH + k] += acc[1];
-          gp[gw3 + k + 8] += acc[2];
-          gp[gw3 + NH + k + 8] += acc[3];
+          put(gw3 + k, acc[0]);
+          put(gw3 + NH + k, acc[1]);
+          put(gw3 + k + 8, acc[2]);
+          put(gw3 + NH + k + 8, acc[3]);
           if (warp == 0 && g == 0) {
-            gp[gb3] += accb[0];
-            gp[gb3 + 1] += accb[1];
+            put(gb3, accb[0]);
+            put(gb3 + 1, accb[1]);
           }
         }
       }
       __syncthreads();
     }
 
-    /* every CTA's partial gradient is complete and visible cluster-wide */
-    cluster.sync();
-    /* the next step's first tile: its global loads overlap the reduction's remote loads */
+    /* every CTA's partial gradient is complete and visible cluster-wide after this barrier; meanwhile the next
+     * step's first tile and what the update needs of this step alone */
+    auto grads = cluster.barrier_arrive();
     prefetched = step + 1 < total_steps && my0 < my1;
     if (prefetched) gather(step + 1, my0);
     const int tstep = step + 1;
     const float lr = tp.lr * (epoch < tp.epochs / 2 ? 1.f
                                                      : 0.1f + 0.9f * (float)(tp.epochs - epoch) / (tp.epochs / 2 + 1));
     const float c1 = 1.f - powf(b1, (float)tstep), c2 = 1.f - powf(b2, (float)tstep);
-    for (int i = lo + tid; i < hi; i += blockDim.x) {
+    cluster.barrier_wait(std::move(grads));
+#pragma unroll
+    for (int u = 0; u < TU; ++u) {
+      const int i = lo + tid + u * TT;
+      if (i >= hi) break;
       float part[CSIZE];
 #pragma unroll
       for (int q = 0; q < CSIZE; ++q) part[q] = cluster.map_shared_rank(gp, q)[i]; /* all loads in flight */
       float gs = 0.f;
 #pragma unroll
       for (int q = 0; q < CSIZE; ++q) gs += part[q];
-      const ParamSlot s = param_slot(i, nin, nh, ldx);
+      const ParamSlot& s = slot[u];
       if (tp.grad_only) {
         if (s.ext >= 0) tp.grad[s.ext] = gs;
         continue;
@@ -779,7 +802,7 @@ static int launch_train(ode_handle* h, const TrainParams& tp, cudaStream_t s, in
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(csize, 1, 1);
-    cfg.blockDim = dim3(TW * 32, 1, 1);
+    cfg.blockDim = dim3(TT, 1, 1);
     cfg.dynamicSmemBytes = L.total;
     cfg.stream = s;
     cfg.attrs = attr;
