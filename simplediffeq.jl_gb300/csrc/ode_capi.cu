@@ -269,23 +269,24 @@ const char* entry_kind(int alg, int sched, int64_t nsave) {
   return nsave > 0 ? "staged" : "persistent";
 }
 
-/* Fixed-step Tsit5 on an ensemble of fewer warps than half the GPU's SM
+/* Fixed-step Tsit5, RK4 or Euler on an ensemble of fewer warps than half the GPU's SM
  * sub-partitions (FP64, final states or every-step output, state output):
  * the kernel that spreads a trajectory's components over the warps of a
- * block (run_fixed_split), one block of 32 * dim threads per 32 trajectories.
+ * block (run_fixed_split, run_onestep_split), one block of 32 * dim threads per 32 trajectories.
  * Only for right-hand sides whose components are separate expressions (each
  * warp computes its own); one with shared work, like Kuramoto's sums of
  * sines, would repeat that work in every warp. */
 bool use_fixed_split(const ode_handle* h, const ode_solve_args* a) {
   const bool separable = a->rhs == ODE_RHS_LORENZ || a->rhs == ODE_RHS_VANDERPOL || a->rhs == ODE_RHS_LINEAR;
-  return a->alg == ODE_ALG_TSIT5 && separable && a->nsave == 0 && a->output == ODE_OUTPUT_STATE &&
+  return (a->alg == ODE_ALG_TSIT5 || is_onestep(a->alg)) && separable && a->nsave == 0 && a->output == ODE_OUTPUT_STATE &&
          a->precision == ODE_FP64 && a->controller != ODE_CTRL_REF && a->dim >= 2 && a->dim <= 8 &&
          (a->n + 31) / 32 <= (int64_t)h->nsm * 2;
 }
 
 /* entry_kind, with the component-split fixed-step kernel where it applies */
 const char* kernel_kind(const ode_handle* h, const ode_solve_args* a, int sched) {
-  return use_fixed_split(h, a) ? "fixedsplit" : entry_kind(a->alg, sched, a->nsave);
+  if (use_fixed_split(h, a)) return is_onestep(a->alg) ? "onestepsplit" : "fixedsplit";
+  return entry_kind(a->alg, sched, a->nsave);
 }
 
 int kernel_kind_id(const char* k) {
@@ -293,7 +294,7 @@ int kernel_kind_id(const char* k) {
   if (!std::strcmp(k, "staged")) return ODE_KERNEL_STAGED;
   if (!std::strcmp(k, "fixed")) return ODE_KERNEL_FIXED;
   if (!std::strcmp(k, "fixedsplit")) return ODE_KERNEL_FIXEDSPLIT;
-  if (!std::strcmp(k, "onestep")) return ODE_KERNEL_ONESTEP;
+  if (!std::strcmp(k, "onestep") || !std::strcmp(k, "onestepsplit")) return ODE_KERNEL_ONESTEP;
   return ODE_KERNEL_PLAIN;
 }
 
