@@ -214,7 +214,10 @@ enum {
   ODE_KERNEL_FIXED = 3,      /* fixed step, one thread per trajectory */
   ODE_KERNEL_FIXEDSPLIT = 4, /* fixed-step Tsit5 with a trajectory's components over the warps of a block
                                 (FP64 ensembles of at most 2 x SMs warps, separable right-hand side) */
-  ODE_KERNEL_ONESTEP = 5     /* RK4 / Euler, one thread per trajectory */
+  ODE_KERNEL_ONESTEP = 5,    /* RK4 / Euler, one thread per trajectory, or like ODE_KERNEL_FIXEDSPLIT */
+  ODE_KERNEL_ADAPTIVESPLIT = 6 /* adaptive Tsit5 under the persistent schedules with a trajectory's components over
+                                the warps of a block (FP64 ensembles of a warp a component for every SM
+                                sub-partition, separable right-hand side) */
 };
 
 /* Bounds-check mode (debugging; compute-sanitizer stands in for nothing

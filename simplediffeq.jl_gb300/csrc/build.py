@@ -51,6 +51,7 @@ GROUPS = {
     # Van der Pol, AVern9 on the restricted three-body problem, ATsit5 on Kuramoto-12
     "lorenz": [("tsit5", "fixed", "lorenz", 3, "fp64"),
                ("tsit5", "fixedsplit", "lorenz", 3, "fp64"),
+               ("atsit5", "adaptivesplit", "lorenz", 3, "fp64"),
                ("atsit5", "plain", "lorenz", 3, "fp64"),
                ("atsit5", "persistent", "lorenz", 3, "fp64")],
     "lorenz_staged": [("atsit5", "staged", "lorenz", 3, "fp64")],

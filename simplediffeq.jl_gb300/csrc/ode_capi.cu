@@ -269,6 +269,9 @@ const char* entry_kind(int alg, int sched, int64_t nsave) {
   return nsave > 0 ? "staged" : "persistent";
 }
 
+/* the ensemble's size: while autotuning, of the whole one and not the sample */
+int64_t ensemble_size(const ode_handle* h, const ode_solve_args* a) { return h->tune_n > 0 ? h->tune_n : a->n; }
+
 /* Fixed-step Tsit5, RK4 or Euler on an ensemble of fewer warps than half the GPU's SM
  * sub-partitions (FP64, final states or every-step output, state output):
  * the kernel that spreads a trajectory's components over the warps of a
@@ -283,13 +286,33 @@ bool use_fixed_split(const ode_handle* h, const ode_solve_args* a) {
          (a->n + 31) / 32 <= (int64_t)h->nsm * 2;
 }
 
-/* entry_kind, with the component-split fixed-step kernel where it applies */
+/* Adaptive Tsit5 under the persistent schedules, for ensembles small enough
+ * that a warp for every component of 32 trajectories still has an SM
+ * sub-partition to itself (run_adaptive_split; with more than four components
+ * the sub-partitions share evenly): a lone warp's attempt is its FP64
+ * instructions at one in 64 cycles, and D warps share them.  Time of the one-
+ * thread-per-trajectory kernel over this one's, Lorenz without and with 100
+ * save points: 1 trajectory 1.55 and 1.31, 32 1.55 and 1.28, 500 1.70 and 1.26,
+ * 2,000 1.59 and 1.18, 4,800 (150 blocks for 152 SMs) 1.26 and 1.03; 6,400, some
+ * SMs with two blocks, 1.17 and 0.86.  Linear, 20 save points, 2,000: dimension
+ * 4 1.54, dimension 2 1.15. */
+bool use_adaptive_split(const ode_handle* h, const ode_solve_args* a, int sched) {
+  const bool separable = a->rhs == ODE_RHS_LORENZ || a->rhs == ODE_RHS_VANDERPOL || a->rhs == ODE_RHS_LINEAR;
+  return a->alg == ODE_ALG_ATSIT5 && sched != ODE_SCHED_PLAIN && separable && a->output == ODE_OUTPUT_STATE &&
+         a->precision == ODE_FP64 && a->controller != ODE_CTRL_REF && a->dim >= 2 && a->dim <= 8 &&
+         !h->bounds_check &&
+         (ensemble_size(h, a) + 31) / 32 <= (int64_t)(a->dim <= 4 ? h->nsm * (4 / a->dim) : h->nsm * 4 / a->dim);
+}
+
+/* entry_kind, with the component-split kernels where they apply */
 const char* kernel_kind(const ode_handle* h, const ode_solve_args* a, int sched) {
+  if (use_adaptive_split(h, a, sched)) return "adaptivesplit";
   if (use_fixed_split(h, a)) return is_onestep(a->alg) ? "onestepsplit" : "fixedsplit";
   return entry_kind(a->alg, sched, a->nsave);
 }
 
 int kernel_kind_id(const char* k) {
+  if (!std::strcmp(k, "adaptivesplit")) return ODE_KERNEL_ADAPTIVESPLIT;
   if (!std::strcmp(k, "persistent")) return ODE_KERNEL_PERSISTENT;
   if (!std::strcmp(k, "staged")) return ODE_KERNEL_STAGED;
   if (!std::strcmp(k, "fixed")) return ODE_KERNEL_FIXED;
@@ -355,8 +378,7 @@ bool crowded(const ode_handle* h, const ode_solve_args* a) {
   if ((a->alg != ODE_ALG_ATSIT5 && a->alg != ODE_ALG_AVERN7) || a->precision != ODE_FP64 ||
       a->controller == ODE_CTRL_REF)
     return false;
-  if (h->tune_crowded >= 0) return h->tune_crowded != 0;
-  return a->n > (int64_t)h->nsm * 4 * (a->alg == ODE_ALG_AVERN7 && a->nsave > 0 ? 160 : 64);
+  return ensemble_size(h, a) > (int64_t)h->nsm * 4 * (a->alg == ODE_ALG_AVERN7 && a->nsave > 0 ? 160 : 64);
 }
 
 /* Whether its kernel keeps the stages in shared memory and forms their linear
@@ -1103,7 +1125,7 @@ int solve_impl(ode_handle* h, const ode_solve_args* a, ode_solve_out* o, ode_sol
   int launches = 0;
   unsigned gridx;
   int block = block_of(h, fn);
-  if (use_fixed_split(h, a)) {
+  if (use_fixed_split(h, a) || use_adaptive_split(h, a, sched)) {
     block = 32 * D;  /* D warps per 32 trajectories */
     gridx = (unsigned)((n + 31) / 32);
   } else if (sched == ODE_SCHED_PLAIN) {
@@ -1675,11 +1697,11 @@ int ode_autotune(ode_handle* h, const ode_solve_args* a, int64_t sample, ode_tun
   to.us = dus;
   to.u_final = duf;
   /* the whole ensemble's kernel is tuned, whatever the sample's size would choose */
-  struct TuneCrowded {
+  struct TuneSize {
     ode_handle* h;
-    ~TuneCrowded() { h->tune_crowded = -1; }
-  } tune_crowded{h};
-  h->tune_crowded = crowded(h, a);
+    ~TuneSize() { h->tune_n = 0; }
+  } tune_size{h};
+  h->tune_n = n;
   const bool ic = use_integer_pipe(h, &ta, ta.schedule);
   const std::string key = kernel_key(h, &ta, ta.schedule);
   /* the baseline is the kernel an untuned handle would run */

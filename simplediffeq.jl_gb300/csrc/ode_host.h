@@ -83,7 +83,7 @@ struct ode_handle {
   unsigned long long graph_tick = 0;
   gbode::Model* model = nullptr;
   bool bounds_check = false;  /* ode_set_bounds_check */
-  int tune_crowded = -1;      /* while autotuning: whether the crowded kernels are tuned (-1: by the size) */
+  int64_t tune_n = 0;         /* while autotuning: the whole ensemble's size */
 };
 
 namespace gbode {

@@ -2943,6 +2943,176 @@ __device__ __forceinline__ void run_fixed_split(const KParams& P) {
   FixedSplitTsit5<PR, D, F>::template dispatch<0>(P, xb, (int)(threadIdx.x >> 5));
 }
 
+/* ------------------------------------------------------------------ adaptive Tsit5, components over warps */
+/* The same split for small adaptive ensembles.  Lane l of warp c works on
+ * component c of trajectory 32 * blockIdx.x + l: its stages and error
+ * estimate, exchanging the stage inputs; the proposal and the error estimate
+ * of every component go to all D warps, which each run the norm and the
+ * controller (adaptive_try), so that all hold the same state, step and
+ * decisions bit for bit.  Save points are interpolated and stored by
+ * component; what else a trajectory writes, warp 0 writes.  A lane whose
+ * trajectory has ended runs on without effect until the block's last one
+ * ends, so every lane meets every barrier. */
+template <class PR, int D, class F>
+struct AdaptiveSplitTsit5 {
+  typedef typename PR::R R;
+  typedef typename PR::T T;
+  typedef MTsit5<PR, 1, F> M1; /* one component's dense output */
+  typedef FixedSplitTsit5<PR, D, F> FS;
+
+  /* the component's stages, and every component's proposal and error estimate */
+  struct Own {
+    R k[7][1];
+    R nh[D], e[D];
+  };
+  /* what adaptive_try calls: the attempt is made before it */
+  struct Method {
+    enum { NK = 7, FSAL = 1, DTMIN_1F7 = 0, DENSE_F = 0 };
+    __device__ static __forceinline__ void attempt(const F&, const R (&)[D], const R (&)[D], T, T, const Own& k,
+                                                   R (&nh)[D], R (&nc)[D], R (&e)[D], bool) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        nh[d] = k.nh[d];
+        nc[d] = (R)0;
+        e[d] = k.e[d];
+      }
+    }
+  };
+
+  __device__ static __forceinline__ bool block_any(bool x) {
+    int any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbarrier.red.or.pred q, 1, %2, p;\n\t"
+                 "selp.s32 %0, 1, 0, q;\n\t}"
+                 : "=r"(any) : "r"((int)x), "r"(32 * D) : "memory");
+    return any != 0;
+  }
+
+  template <int C>
+  __device__ static __forceinline__ void attempt(const F& f, R (*xb)[D][32], int& b, int lane, const R (&uh)[D], T t,
+                                                 T dt, Own& o) {
+#define C5(x) CB<R>::t5(tsit5_##x)
+#define C5T(x) CB<T>::t5(tsit5_##x)
+    R (&k)[7][1] = o.k;
+    const R u[1] = {uh[C]}, u0[1] = {(R)0}, h = (R)dt;
+    R tmp[1], s[1], nh[1], nc[1], full[D];
+    const R a = (R)(dt * C5T(a21));
+    tmp[0] = fmaR(a, k[0][0], u[0]);
+    FS::exchange(xb, b, C, lane, tmp[0], full);
+    k[1][0] = FS::template rhs<C>(f, full, stime(t, C5T(c1), dt));
+    lc(s, C5(a31), k[0], C5(a32), k[1]);
+    axpy(tmp, u, h, s);
+    FS::exchange(xb, b, C, lane, tmp[0], full);
+    k[2][0] = FS::template rhs<C>(f, full, stime(t, C5T(c2), dt));
+    lc(s, C5(a41), k[0], C5(a42), k[1], C5(a43), k[2]);
+    axpy(tmp, u, h, s);
+    FS::exchange(xb, b, C, lane, tmp[0], full);
+    k[3][0] = FS::template rhs<C>(f, full, stime(t, C5T(c3), dt));
+    lc(s, C5(a51), k[0], C5(a52), k[1], C5(a53), k[2], C5(a54), k[3]);
+    axpy(tmp, u, h, s);
+    FS::exchange(xb, b, C, lane, tmp[0], full);
+    k[4][0] = FS::template rhs<C>(f, full, stime(t, C5T(c4), dt));
+    lc(s, C5(a61), k[0], C5(a62), k[1], C5(a63), k[2], C5(a64), k[3], C5(a65), k[4]);
+    axpy(tmp, u, h, s);
+    FS::exchange(xb, b, C, lane, tmp[0], full);
+    k[5][0] = FS::template rhs<C>(f, full, t + dt);
+    lc(s, C5(a71), k[0], C5(a72), k[1], C5(a73), k[2], C5(a74), k[3], C5(a75), k[4], C5(a76), k[5]);
+    state_update<PR, 1>(u, u0, h, s, nh, nc);
+    FS::exchange(xb, b, C, lane, nh[0], o.nh);
+    k[6][0] = FS::template rhs<C>(f, o.nh, t + dt);
+    lc(s, C5(btilde1), k[0], C5(btilde2), k[1], C5(btilde3), k[2], C5(btilde4), k[3], C5(btilde5), k[4], C5(btilde6),
+       k[5], C5(btilde7), k[6]);
+    FS::exchange(xb, b, C, lane, ErrUnscaled<R>::value ? s[0] : h * s[0], o.e);
+#undef C5
+#undef C5T
+  }
+
+  template <int C>
+  __device__ static __forceinline__ void run(const KParams& P0, R (*xb)[D][32]) {
+    KParams P = P0;
+    if (C != 0) {
+      /* warp 0 writes these */
+      P.u_final = 0;
+      P.t_final = 0;
+      P.retcode = 0;
+      P.naccept = 0;
+      P.nreject = 0;
+      P.dt_first = 0;
+      P.ev_t = 0;
+      P.stats = 0;
+      P.us = 0;
+    }
+    const int lane = threadIdx.x & 31;
+    const long long i = (long long)blockIdx.x * 32 + lane;
+    Totals tot = {0, 0, 0};
+    Lane<PR, D, F, 7, Own> l;
+    bool active = i < P.n;
+    /* lanes past n run trajectory 0 without effect */
+    if (active) {
+      lane_load(P, i, l);
+      if (!(l.t < (T)P.tf)) {
+        lane_finish(P, l, RET_DEFAULT, tot);
+        active = false;
+      }
+    } else {
+      KParams Q = P;
+      Q.u_final = 0;
+      Q.ev_t = 0;
+      Q.us = 0;
+      lane_load(Q, 0, l);
+    }
+    l.k.k[0][0] = FS::template rhs<C>(l.f, l.uh, l.t);
+    int b = 0;
+    /* the block goes on while any of its threads has work, so that its warps meet the same barriers */
+    while (block_any(active)) {
+      __syncwarp();
+      attempt<C>(l.f, xb, b, lane, l.uh, l.t, l.dt, l.k);
+      if (!active) continue;
+      R nh[D], nc[D];
+      Accepted<T> st;
+      const int r = adaptive_try<Method>(P, l, tot, nh, nc, st);
+      if (r == TRY_STOPPED) active = false;
+      if (r != TRY_ACCEPTED) continue;
+      T inv_dt = (T)0;
+      if (l.cur < P.nsave && t_le<PR>(P.saveat[l.cur], l.t)) inv_dt = recip(st.dtold);
+      while (l.cur < P.nsave && t_le<PR>(P.saveat[l.cur], l.t)) {
+        const T theta = theta_of((T)P.saveat[l.cur], st.told, st.dtold, inv_dt);
+        const R u[1] = {l.uh[C]}, uc[1] = {(R)0};
+        double v[1];
+        M1::dense(l.f, u, uc, st.told, l.t, st.dtold, theta, l.k.k, v);
+        if (P0.us && GBODE_CHECK(P, l.idx >= 0 && l.idx < P.n && l.cur >= 0 && l.cur < P.nsave, CHK_SAVE))
+          *us_at(P0, l.cur, C, l.idx) = v[0];
+        l.cur += 1;
+        l.ninterp += 1;
+      }
+#pragma unroll
+      for (int d = 0; d < D; ++d) l.uh[d] = nh[d];
+      l.k.k[0][0] = l.k.k[6][0];
+      store_step<PR, D>(P, l, l.nacc);
+      if (!t_lt<PR>(l.t, P.tf)) {
+        lane_finish(P, l, RET_DEFAULT, tot);
+        active = false;
+      }
+    }
+    flush_totals(P, tot);
+  }
+
+  /* the warp's component as a compile-time constant */
+  template <int C>
+  __device__ static __forceinline__ void dispatch(const KParams& P, R (*xb)[D][32], int w) {
+    if constexpr (C < D) {
+      if (w == C) run<C>(P, xb);
+      else dispatch<C + 1>(P, xb, w);
+    }
+  }
+};
+
+template <class PR, int D, class F>
+__device__ __forceinline__ void run_adaptive_split(const KParams& P) {
+  typedef typename PR::R R;
+  __shared__ R xb[2][D][32];
+  AdaptiveSplitTsit5<PR, D, F>::template dispatch<0>(P, xb, (int)(threadIdx.x >> 5));
+}
+
 /* ------------------------------------------------------------------ RK4 and Euler, components over warps */
 /* The same split for the one-step methods (M = MRK4 or MEuler): per component
  * the operations of M::step and run_onestep in the same order.  4,001
@@ -3164,7 +3334,11 @@ __device__ __forceinline__ void run_onestep(const KParams& P) {
   extern "C" __global__ void __launch_bounds__(GBODE_BLOCK) NAME(gbode::KParams P) {                \
     gbode::run_onestep<M<PR, RHS::D, RHS>, PR, RHS::D, RHS>(P);                              \
   }
-/* RK4 and Euler the same way */
+/* adaptive Tsit5, RK4 and Euler the same way */
+#define GBODE_ENTRY_adaptivesplit(NAME, M, PR, RHS)                                          \
+  extern "C" __global__ void __launch_bounds__(32 * RHS::D) NAME(gbode::KParams P) {              \
+    gbode::run_adaptive_split<PR, RHS::D, RHS>(P);                                          \
+  }
 #define GBODE_ENTRY_onestepsplit(NAME, M, PR, RHS)                                           \
   extern "C" __global__ void __launch_bounds__(32 * RHS::D) NAME(gbode::KParams P) {              \
     gbode::run_onestep_split<M<PR, RHS::D, RHS>, PR, RHS::D, RHS>(P);                        \
