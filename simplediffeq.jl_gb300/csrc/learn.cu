@@ -339,13 +339,13 @@ struct TrainLayout {
     b1 = take(NH * 4);
     b2 = take(NH * 4);
     b3 = take(W3ROWS * 4);
-    xs = take((size_t)TROWS * ldx * 2);
+    xs = take((size_t)TROWS * ldx * 2 * 2); /* this tile's and the next one's */
     h1 = take((size_t)TROWS * LDH * 2);
     h2 = take((size_t)TROWS * LDH * 2);
     d1 = take((size_t)TROWS * LDH * 2);
     d2 = take((size_t)TROWS * LDH * 2);
     dout = take((size_t)TROWS * 8 * 2);
-    ys = take((size_t)TROWS * 2 * 4);
+    ys = take((size_t)TROWS * 2 * 4 * 2);
     gp = take((size_t)P * 4);
     om = take((size_t)S * 4);
     ov = take((size_t)S * 4);
@@ -441,11 +441,16 @@ __device__ __forceinline__ uint32_t permute(uint32_t i, const Perm& p) {
  * comment).  Grid = the cluster: CSIZE CTAs of TT threads.
  *
  * A step is a chain of small dependent products between two cluster barriers,
- * bound by latency.  What does not depend on the other CTAs (the next tile's
- * gather, the step's Adam constants) runs between a barrier's arrive and its
+ * bound by latency (1,920 steps of 1,024 samples, six inputs, 64 of them in each
+ * of 16 CTAs; cycles a step: forward and backward 3,400, weight gradients 2,570,
+ * the first barrier 1,480, the update 3,490, the second barrier 1,800).  What
+ * does not depend on the other CTAs runs between a barrier's arrive and its
  * wait, a tile's first gradient is stored, not added to a zeroed array, and
- * where a parameter lies is worked out once, not every step: 15.1 to 13.1 ms for
- * 1,920 steps of 1,024 samples. */
+ * where a parameter lies is worked out once, not every step: 15.1 to 13.1 ms.
+ * The two warps without a part in the products gather the next tile into a
+ * second buffer while the current one is worked on (its permutation walk and
+ * loads, 3,200 cycles, were between the barriers), and one loop over the
+ * samples carries all three weight-gradient products: 13.1 to 11.6 ms. */
 template <int KIN, int CSIZE>
 __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
   constexpr int csize = CSIZE;
@@ -464,13 +469,13 @@ __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
   net.b2 = (float*)(smem + L.b2);
   net.b3 = (float*)(smem + L.b3);
   net.ldx = L.ldx;
-  __nv_bfloat16* xs = (__nv_bfloat16*)(smem + L.xs);
+  __nv_bfloat16* const xs2 = (__nv_bfloat16*)(smem + L.xs);
   __nv_bfloat16* h1s = (__nv_bfloat16*)(smem + L.h1);
   __nv_bfloat16* h2s = (__nv_bfloat16*)(smem + L.h2);
   __nv_bfloat16* d1s = (__nv_bfloat16*)(smem + L.d1);
   __nv_bfloat16* d2s = (__nv_bfloat16*)(smem + L.d2);
   __nv_bfloat16* douts = (__nv_bfloat16*)(smem + L.dout);
-  float* ys = (float*)(smem + L.ys);
+  float* const ys2 = (float*)(smem + L.ys);
   float* gp = (float*)(smem + L.gp);
   float* om = (float*)(smem + L.om);
   float* ov = (float*)(smem + L.ov);
@@ -502,27 +507,32 @@ __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
   const int total_steps = tp.grad_only ? 1 : tp.epochs * tp.steps_per_epoch;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
 
-  /* the tile of step `st` starting at batch row r0: features to bf16, targets,
-   * zero rows beyond the batch */
-  auto gather = [&](int st, int r0) {
+  /* the tile of step `st` starting at batch row r0 into buffer `to`: features to bf16, targets, zero rows beyond the
+   * batch.  Threads `from` and up take a row each. */
+  auto gather = [&](int st, int r0, int to, int from) {
     const int valid = min(TROWS, my1 - r0);
     const int sie = tp.grad_only ? 0 : st % tp.steps_per_epoch;
     const Perm perm = make_perm((uint32_t)tp.nb, tp.seed_lo, tp.seed_hi,
                                 (uint32_t)(tp.grad_only ? 0 : st / tp.steps_per_epoch));
     const int rows = (valid + 15) & ~15; /* what the products read */
-    for (int i = tid; i < rows * 2; i += blockDim.x) {
-      const int s = i >> 1, half = i & 1;
+    __nv_bfloat16* const xs = xs2 + to * TROWS * ldx;
+    float* const ys = ys2 + to * TROWS * 2;
+    for (int s = tid - from; s < rows; s += TT - from) {
       int idx = -1;
       if (s < valid) {
         const uint32_t pos = (uint32_t)(sie * tp.batch + r0 + s);
         idx = tp.grad_only ? (int)pos : (int)permute(pos, perm);
       }
-      for (int f = half; f < ldx - 8; f += 2)
+#pragma unroll
+      for (int f = 0; f < KIN * 16; ++f)
         xs[s * ldx + f] = __float2bfloat16((idx >= 0 && f < nin) ? tp.X[(size_t)idx * nin + f] : 0.f);
-      ys[s * 2 + half] = idx >= 0 ? tp.Y[(size_t)idx * NOUT + half] : 0.f;
+#pragma unroll
+      for (int q = 0; q < NOUT; ++q) ys[s * 2 + q] = idx >= 0 ? tp.Y[(size_t)idx * NOUT + q] : 0.f;
     }
   };
-  bool prefetched = false; /* the step's first tile was gathered during the previous step's reduction */
+  int cur = 0; /* the current tile's buffer */
+  if (my0 < my1) gather(0, my0, 0, 0);
+  __syncthreads();
 
   for (int step = 0; step < total_steps; ++step) {
     const int epoch = tp.grad_only ? 0 : step / tp.steps_per_epoch;
@@ -533,189 +543,179 @@ __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
     for (int r0 = my0; r0 < my1; r0 += TROWS) {
       const int valid = min(TROWS, my1 - r0);
       const int kmax = (valid + 15) >> 4;
-      if (!(prefetched && r0 == my0)) gather(step, r0);
-      __syncthreads();
-      /* per warp: forward, output deltas, backward through both hidden layers */
-      const int wr = warp * 16;
-      if (wr < valid) {
-        float out[4];
-        uint32_t mask1, mask2;
-        warp_forward<KIN, true>(net, xs, wr, out, h1s, h2s, mask1, mask2);
-        float dg0 = 0.f, dg1 = 0.f, dh0 = 0.f, dh1 = 0.f, lsum = 0.f;
-        if (t == 0) {
-          if (wr + g < valid) {
-            const float e0 = out[0] - ys[(wr + g) * 2], e1 = out[1] - ys[(wr + g) * 2 + 1];
-            lsum = e0 * e0 * inv_b + e1 * e1 * inv_b;
-            dg0 = bf16r(2.f * e0 * inv_b);
-            dg1 = bf16r(2.f * e1 * inv_b);
+      const __nv_bfloat16* const xs = xs2 + cur * TROWS * ldx;
+      const float* const ys = ys2 + cur * TROWS * 2;
+      if (warp >= TW) {
+        /* the warps without a part in the products gather the next tile meanwhile */
+        const bool more = r0 + TROWS < my1;
+        if (more || step + 1 < total_steps) gather(more ? step : step + 1, more ? r0 + TROWS : my0, cur ^ 1, 32 * TW);
+      } else {
+        /* per warp: forward, output deltas, backward through both hidden layers */
+        const int wr = warp * 16;
+        if (wr < valid) {
+          float out[4];
+          uint32_t mask1, mask2;
+          warp_forward<KIN, true>(net, xs, wr, out, h1s, h2s, mask1, mask2);
+          float dg0 = 0.f, dg1 = 0.f, dh0 = 0.f, dh1 = 0.f, lsum = 0.f;
+          if (t == 0) {
+            if (wr + g < valid) {
+              const float e0 = out[0] - ys[(wr + g) * 2], e1 = out[1] - ys[(wr + g) * 2 + 1];
+              lsum = e0 * e0 * inv_b + e1 * e1 * inv_b;
+              dg0 = bf16r(2.f * e0 * inv_b);
+              dg1 = bf16r(2.f * e1 * inv_b);
+            }
+            if (wr + g + 8 < valid) {
+              const float e0 = out[2] - ys[(wr + g + 8) * 2], e1 = out[3] - ys[(wr + g + 8) * 2 + 1];
+              lsum += e0 * e0 * inv_b + e1 * e1 * inv_b;
+              dh0 = bf16r(2.f * e0 * inv_b);
+              dh1 = bf16r(2.f * e1 * inv_b);
+            }
+            *reinterpret_cast<uint32_t*>(douts + (wr + g) * 8) = pack_bf16(dg0, dg1);
+            *reinterpret_cast<uint32_t*>(douts + (wr + g + 8) * 8) = pack_bf16(dh0, dh1);
           }
-          if (wr + g + 8 < valid) {
-            const float e0 = out[2] - ys[(wr + g + 8) * 2], e1 = out[3] - ys[(wr + g + 8) * 2 + 1];
-            lsum += e0 * e0 * inv_b + e1 * e1 * inv_b;
-            dh0 = bf16r(2.f * e0 * inv_b);
-            dh1 = bf16r(2.f * e1 * inv_b);
-          }
-          *reinterpret_cast<uint32_t*>(douts + (wr + g) * 8) = pack_bf16(dg0, dg1);
-          *reinterpret_cast<uint32_t*>(douts + (wr + g + 8) * 8) = pack_bf16(dh0, dh1);
-        }
-        lsum += __shfl_xor_sync(0xffffffffu, lsum, 4);
-        lsum += __shfl_xor_sync(0xffffffffu, lsum, 8);
-        lsum += __shfl_xor_sync(0xffffffffu, lsum, 16);
-        if (lane == 0) atomicAdd(sloss, lsum);
-        const int src = lane & ~3;
-        dg0 = __shfl_sync(0xffffffffu, dg0, src);
-        dg1 = __shfl_sync(0xffffffffu, dg1, src);
-        dh0 = __shfl_sync(0xffffffffu, dh0, src);
-        dh1 = __shfl_sync(0xffffffffu, dh1, src);
-        /* d2 = W3^T dout (bf16 operands, both products exact in fp32), masked by layer 2's ReLU */
-        uint32_t ad[4][4];
-        float acc[8][4];
+          lsum += __shfl_xor_sync(0xffffffffu, lsum, 4);
+          lsum += __shfl_xor_sync(0xffffffffu, lsum, 8);
+          lsum += __shfl_xor_sync(0xffffffffu, lsum, 16);
+          if (lane == 0) atomicAdd(sloss, lsum);
+          const int src = lane & ~3;
+          dg0 = __shfl_sync(0xffffffffu, dg0, src);
+          dg1 = __shfl_sync(0xffffffffu, dg1, src);
+          dh0 = __shfl_sync(0xffffffffu, dh0, src);
+          dh1 = __shfl_sync(0xffffffffu, dh1, src);
+          /* d2 = W3^T dout (bf16 operands, both products exact in fp32), masked by layer 2's ReLU */
+          uint32_t ad[4][4];
+          float acc[8][4];
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const int j = nt * 8 + 2 * t;
-          const float w0a = __bfloat162float(net.w3[j]), w0b = __bfloat162float(net.w3[j + 1]);
-          const float w1a = __bfloat162float(net.w3[LDH + j]), w1b = __bfloat162float(net.w3[LDH + j + 1]);
-          acc[nt][0] = (mask2 >> (nt * 4 + 0) & 1u) ? fmaf(w0a, dg0, w1a * dg1) : 0.f;
-          acc[nt][1] = (mask2 >> (nt * 4 + 1) & 1u) ? fmaf(w0b, dg0, w1b * dg1) : 0.f;
-          acc[nt][2] = (mask2 >> (nt * 4 + 2) & 1u) ? fmaf(w0a, dh0, w1a * dh1) : 0.f;
-          acc[nt][3] = (mask2 >> (nt * 4 + 3) & 1u) ? fmaf(w0b, dh0, w1b * dh1) : 0.f;
-        }
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          ad[kk][0] = pack_bf16(acc[2 * kk][0], acc[2 * kk][1]);
-          ad[kk][1] = pack_bf16(acc[2 * kk][2], acc[2 * kk][3]);
-          ad[kk][2] = pack_bf16(acc[2 * kk + 1][0], acc[2 * kk + 1][1]);
-          ad[kk][3] = pack_bf16(acc[2 * kk + 1][2], acc[2 * kk + 1][3]);
-          *reinterpret_cast<uint32_t*>(d2s + (wr + g) * LDH + kk * 16 + 2 * t) = ad[kk][0];
-          *reinterpret_cast<uint32_t*>(d2s + (wr + g + 8) * LDH + kk * 16 + 2 * t) = ad[kk][1];
-          *reinterpret_cast<uint32_t*>(d2s + (wr + g) * LDH + kk * 16 + 8 + 2 * t) = ad[kk][2];
-          *reinterpret_cast<uint32_t*>(d2s + (wr + g + 8) * LDH + kk * 16 + 8 + 2 * t) = ad[kk][3];
-        }
-        /* d1 = W2^T d2, masked by layer 1's ReLU */
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-          for (int np = 0; np < 4; ++np) {
-            uint32_t b[4];
-            ldsm_x4_t(b, net.w2 + (kk * 16 + (mi & 1) * 8 + ri) * LDH + np * 16 + (mi >> 1) * 8);
-            mma_bf16(acc[2 * np], ad[kk], b[0], b[1]);
-            mma_bf16(acc[2 * np + 1], ad[kk], b[2], b[3]);
+          for (int nt = 0; nt < 8; ++nt) {
+            const int j = nt * 8 + 2 * t;
+            const float w0a = __bfloat162float(net.w3[j]), w0b = __bfloat162float(net.w3[j + 1]);
+            const float w1a = __bfloat162float(net.w3[LDH + j]), w1b = __bfloat162float(net.w3[LDH + j + 1]);
+            acc[nt][0] = (mask2 >> (nt * 4 + 0) & 1u) ? fmaf(w0a, dg0, w1a * dg1) : 0.f;
+            acc[nt][1] = (mask2 >> (nt * 4 + 1) & 1u) ? fmaf(w0b, dg0, w1b * dg1) : 0.f;
+            acc[nt][2] = (mask2 >> (nt * 4 + 2) & 1u) ? fmaf(w0a, dh0, w1a * dh1) : 0.f;
+            acc[nt][3] = (mask2 >> (nt * 4 + 3) & 1u) ? fmaf(w0b, dh0, w1b * dh1) : 0.f;
           }
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const float v0 = (mask1 >> (nt * 4 + 0) & 1u) ? acc[nt][0] : 0.f;
-          const float v1 = (mask1 >> (nt * 4 + 1) & 1u) ? acc[nt][1] : 0.f;
-          const float v2 = (mask1 >> (nt * 4 + 2) & 1u) ? acc[nt][2] : 0.f;
-          const float v3 = (mask1 >> (nt * 4 + 3) & 1u) ? acc[nt][3] : 0.f;
-          *reinterpret_cast<uint32_t*>(d1s + (wr + g) * LDH + nt * 8 + 2 * t) = pack_bf16(v0, v1);
-          *reinterpret_cast<uint32_t*>(d1s + (wr + g + 8) * LDH + nt * 8 + 2 * t) = pack_bf16(v2, v3);
+          for (int kk = 0; kk < 4; ++kk) {
+            ad[kk][0] = pack_bf16(acc[2 * kk][0], acc[2 * kk][1]);
+            ad[kk][1] = pack_bf16(acc[2 * kk][2], acc[2 * kk][3]);
+            ad[kk][2] = pack_bf16(acc[2 * kk + 1][0], acc[2 * kk + 1][1]);
+            ad[kk][3] = pack_bf16(acc[2 * kk + 1][2], acc[2 * kk + 1][3]);
+            *reinterpret_cast<uint32_t*>(d2s + (wr + g) * LDH + kk * 16 + 2 * t) = ad[kk][0];
+            *reinterpret_cast<uint32_t*>(d2s + (wr + g + 8) * LDH + kk * 16 + 2 * t) = ad[kk][1];
+            *reinterpret_cast<uint32_t*>(d2s + (wr + g) * LDH + kk * 16 + 8 + 2 * t) = ad[kk][2];
+            *reinterpret_cast<uint32_t*>(d2s + (wr + g + 8) * LDH + kk * 16 + 8 + 2 * t) = ad[kk][3];
+          }
+          /* d1 = W2^T d2, masked by layer 1's ReLU */
+#pragma unroll
+          for (int nt = 0; nt < 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int np = 0; np < 4; ++np) {
+              uint32_t b[4];
+              ldsm_x4_t(b, net.w2 + (kk * 16 + (mi & 1) * 8 + ri) * LDH + np * 16 + (mi >> 1) * 8);
+              mma_bf16(acc[2 * np], ad[kk], b[0], b[1]);
+              mma_bf16(acc[2 * np + 1], ad[kk], b[2], b[3]);
+            }
+#pragma unroll
+          for (int nt = 0; nt < 8; ++nt) {
+            const float v0 = (mask1 >> (nt * 4 + 0) & 1u) ? acc[nt][0] : 0.f;
+            const float v1 = (mask1 >> (nt * 4 + 1) & 1u) ? acc[nt][1] : 0.f;
+            const float v2 = (mask1 >> (nt * 4 + 2) & 1u) ? acc[nt][2] : 0.f;
+            const float v3 = (mask1 >> (nt * 4 + 3) & 1u) ? acc[nt][3] : 0.f;
+            *reinterpret_cast<uint32_t*>(d1s + (wr + g) * LDH + nt * 8 + 2 * t) = pack_bf16(v0, v1);
+            *reinterpret_cast<uint32_t*>(d1s + (wr + g + 8) * LDH + nt * 8 + 2 * t) = pack_bf16(v2, v3);
+          }
         }
-      }
-      __syncthreads();
-      /* weight gradients over the tile's samples (K = samples, operands read transposed); the first tile's are
-       * stored, the others' added */
-      const bool first = r0 == my0;
-      auto put = [&](int i, float v) { gp[i] = first ? v : gp[i] + v; };
-      if (warp < TW) {
-        /* gW2[j][k] = sum_s d2[s][j] h1[s][k]; gb2[j] = sum_s d2[s][j] (ones operand) */
-        const int mt = warp >> 1, nb0 = (warp & 1) * 32;
-        float acc[4][4] = {};
-        float accb[4] = {};
-        const bool bias = (warp & 1) == 0;
+        /* (the gathering warps do not wait here) */
+        asm volatile("barrier.sync 1, %0;" ::"n"(32 * TW) : "memory");
+        /* weight gradients over the tile's samples (K = samples, operands read transposed); the first tile's are
+         * stored, the others' added.  gW2[j][k] = sum_s d2[s][j] h1[s][k] and gW1[j][f] = sum_s d1[s][j] x[s][f] over
+         * all warps, their bias gradients (ones operand) on the warps with the first columns; gW3[q][k] =
+         * sum_s dout[s][q] h2[s][k] as (h2^T dout)[k][q] on warps 4 to 7.  One loop over the samples carries the
+         * products of all three, so that their latencies overlap. */
+        const bool first = r0 == my0;
+        auto put = [&](int i, float v) { gp[i] = first ? v : gp[i] + v; };
+        const int mt2 = warp >> 1, nb0 = (warp & 1) * 32, mt1 = warp & 3, nt1 = warp >> 2;
+        const bool bias2 = (warp & 1) == 0, low = warp < 4;
         const uint32_t ones = g == 0 ? kOnesBf16x2 : 0u;
+        float a2[4][4] = {}, a2b[4] = {}, a1[KIN][4] = {}, a1b[4] = {}, a3[4] = {}, a3b[4] = {};
         for (int ks = 0; ks < kmax; ++ks) {
-          uint32_t a[4];
-          ldsm_x4_t(a, d2s + (ks * 16 + (mi >> 1) * 8 + ri) * LDH + mt * 16 + (mi & 1) * 8);
+          uint32_t a[4], b[2][4], c[4], x[KIN][2];
+          const int ra = ks * 16 + (mi >> 1) * 8 + ri, rb = ks * 16 + (mi & 1) * 8 + ri;
+          ldsm_x4_t(a, d2s + ra * LDH + mt2 * 16 + (mi & 1) * 8);
+          ldsm_x4_t(b[0], h1s + rb * LDH + nb0 + (mi >> 1) * 8);
+          ldsm_x4_t(b[1], h1s + rb * LDH + nb0 + 16 + (mi >> 1) * 8);
+          ldsm_x4_t(c, d1s + ra * LDH + mt1 * 16 + (mi & 1) * 8);
+#pragma unroll
+          for (int r = 0; r < KIN; ++r) ldsm_x2_t(x[r], xs + rb * ldx + (nt1 + 2 * r) * 8);
+          if (!low) {
+            uint32_t h[4], o[2];
+            ldsm_x4_t(h, h2s + ra * LDH + mt1 * 16 + (mi & 1) * 8);
+            ldsm_x2_t(o, douts + rb * 8);
+            mma_bf16(a3, h, o[0], o[1]);
+            const uint32_t onesa[4] = {ones, 0u, ones, 0u};
+            if (warp == 4) mma_bf16(a3b, onesa, o[0], o[1]); /* gb3[q] = sum_s dout[s][q] */
+          }
 #pragma unroll
           for (int np = 0; np < 2; ++np) {
-            uint32_t b[4];
-            ldsm_x4_t(b, h1s + (ks * 16 + (mi & 1) * 8 + ri) * LDH + nb0 + np * 16 + (mi >> 1) * 8);
-            mma_bf16(acc[2 * np], a, b[0], b[1]);
-            mma_bf16(acc[2 * np + 1], a, b[2], b[3]);
+            mma_bf16(a2[2 * np], a, b[np][0], b[np][1]);
+            mma_bf16(a2[2 * np + 1], a, b[np][2], b[np][3]);
           }
-          if (bias) mma_bf16(accb, a, ones, ones);
+#pragma unroll
+          for (int r = 0; r < KIN; ++r) mma_bf16(a1[r], c, x[r][0], x[r][1]);
+          if (bias2) mma_bf16(a2b, a, ones, ones);
+          if (low) mma_bf16(a1b, c, ones, ones);
         }
-        const int gw2 = NH * nin + NH, gb2 = gw2 + NH * NH;
+        const int gw1 = 0, gb1 = NH * nin, gw2 = gb1 + NH, gb2 = gw2 + NH * NH, gw3 = gb2 + NH, gb3 = gw3 + NOUT * NH;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-          const int j = mt * 16 + g, k = nb0 + nt * 8 + 2 * t;
-          put(gw2 + j * NH + k, acc[nt][0]);
-          put(gw2 + j * NH + k + 1, acc[nt][1]);
-          put(gw2 + (j + 8) * NH + k, acc[nt][2]);
-          put(gw2 + (j + 8) * NH + k + 1, acc[nt][3]);
+          const int j = mt2 * 16 + g, k = nb0 + nt * 8 + 2 * t;
+          put(gw2 + j * NH + k, a2[nt][0]);
+          put(gw2 + j * NH + k + 1, a2[nt][1]);
+          put(gw2 + (j + 8) * NH + k, a2[nt][2]);
+          put(gw2 + (j + 8) * NH + k + 1, a2[nt][3]);
         }
-        if (bias && t == 0) {
-          put(gb2 + mt * 16 + g, accb[0]);
-          put(gb2 + mt * 16 + g + 8, accb[2]);
+        if (bias2 && t == 0) {
+          put(gb2 + mt2 * 16 + g, a2b[0]);
+          put(gb2 + mt2 * 16 + g + 8, a2b[2]);
         }
-      }
-      {
-        /* gW1[j][f] = sum_s d1[s][j] x[s][f]; gb1[j] = sum_s d1[s][j] */
-        const int gw1 = 0, gb1 = NH * nin;
-        const uint32_t ones = g == 0 ? kOnesBf16x2 : 0u;
-        for (int id = warp; id < (warp < TW ? 8 * KIN : 0); id += TW) {
-          const int mt = id & 3, nt = id >> 2;
-          float acc[4] = {};
-          float accb[4] = {};
-          const bool bias = nt == 0;
-          for (int ks = 0; ks < kmax; ++ks) {
-            uint32_t a[4], b[2];
-            ldsm_x4_t(a, d1s + (ks * 16 + (mi >> 1) * 8 + ri) * LDH + mt * 16 + (mi & 1) * 8);
-            ldsm_x2_t(b, xs + (ks * 16 + (mi & 1) * 8 + ri) * ldx + nt * 8);
-            mma_bf16(acc, a, b[0], b[1]);
-            if (bias) mma_bf16(accb, a, ones, ones);
-          }
-          const int j = mt * 16 + g, f = nt * 8 + 2 * t;
+#pragma unroll
+        for (int r = 0; r < KIN; ++r) {
+          const int j = mt1 * 16 + g, f = (nt1 + 2 * r) * 8 + 2 * t;
           if (f < nin) {
-            put(gw1 + j * nin + f, acc[0]);
-            put(gw1 + (j + 8) * nin + f, acc[2]);
+            put(gw1 + j * nin + f, a1[r][0]);
+            put(gw1 + (j + 8) * nin + f, a1[r][2]);
           }
           if (f + 1 < nin) {
-            put(gw1 + j * nin + f + 1, acc[1]);
-            put(gw1 + (j + 8) * nin + f + 1, acc[3]);
-          }
-          if (bias && t == 0) {
-            put(gb1 + mt * 16 + g, accb[0]);
-            put(gb1 + mt * 16 + g + 8, accb[2]);
+            put(gw1 + j * nin + f + 1, a1[r][1]);
+            put(gw1 + (j + 8) * nin + f + 1, a1[r][3]);
           }
         }
-      }
-      if (warp < 4) {
-        /* gW3[q][k] = sum_s dout[s][q] h2[s][k] as (h2^T dout)[k][q]; warp 0 also gb3[q] = sum_s dout[s][q] */
-        const int mt = warp;
-        float acc[4] = {};
-        float accb[4] = {};
-        uint32_t onesa[4] = {g == 0 ? kOnesBf16x2 : 0u, 0u, g == 0 ? kOnesBf16x2 : 0u, 0u};
-        for (int ks = 0; ks < kmax; ++ks) {
-          uint32_t a[4], b[2];
-          ldsm_x4_t(a, h2s + (ks * 16 + (mi >> 1) * 8 + ri) * LDH + mt * 16 + (mi & 1) * 8);
-          ldsm_x2_t(b, douts + (ks * 16 + (mi & 1) * 8 + ri) * 8);
-          mma_bf16(acc, a, b[0], b[1]);
-          if (warp == 0) mma_bf16(accb, onesa, b[0], b[1]);
+        if (low && t == 0) {
+          put(gb1 + mt1 * 16 + g, a1b[0]);
+          put(gb1 + mt1 * 16 + g + 8, a1b[2]);
         }
-        const int gw3 = NH * nin + 2 * NH + NH * NH, gb3 = gw3 + NOUT * NH;
-        if (t == 0) {
-          const int k = mt * 16 + g;
-          put(gw3 + k, acc[0]);
-          put(gw3 + NH + k, acc[1]);
-          put(gw3 + k + 8, acc[2]);
-          put(gw3 + NH + k + 8, acc[3]);
-          if (warp == 0 && g == 0) {
-            put(gb3, accb[0]);
-            put(gb3 + 1, accb[1]);
+        if (!low && t == 0) {
+          const int k = mt1 * 16 + g;
+          put(gw3 + k, a3[0]);
+          put(gw3 + NH + k, a3[1]);
+          put(gw3 + k + 8, a3[2]);
+          put(gw3 + NH + k + 8, a3[3]);
+          if (warp == 4 && g == 0) {
+            put(gb3, a3b[0]);
+            put(gb3 + 1, a3b[1]);
           }
         }
       }
       __syncthreads();
+      cur ^= 1;
     }
 
-    /* every CTA's partial gradient is complete and visible cluster-wide after this barrier; meanwhile the next
-     * step's first tile and what the update needs of this step alone */
+    /* every CTA's partial gradient is complete and visible cluster-wide after this barrier; meanwhile what
+     * the update needs of this step alone */
     auto grads = cluster.barrier_arrive();
-    prefetched = step + 1 < total_steps && my0 < my1;
-    if (prefetched) gather(step + 1, my0);
     const int tstep = step + 1;
     const float lr = tp.lr * (epoch < tp.epochs / 2 ? 1.f
                                                      : 0.1f + 0.9f * (float)(tp.epochs - epoch) / (tp.epochs / 2 + 1));
