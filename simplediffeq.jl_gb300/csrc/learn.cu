@@ -20,11 +20,11 @@
  * from one layer to the next and written to shared memory once (bf16) for the
  * weight-gradient products, which run CTA-wide over the tile's samples.
  * Each CTA's partial gradient sits in its shared memory; CTA r owns a slice
- * of the parameters, sums that slice over the cluster through distributed
- * shared memory (fixed order: every run gives the same bits), applies Adam to
- * its fp32 master copy and writes the bf16 weights into every CTA's network.
- * Two cluster barriers a step, no global-memory round trip, no host work
- * between steps.  Samples are drawn per epoch through a keyed Feistel
+ * of the parameters, receives that slice of every CTA's gradient by bulk copies
+ * between shared memories, sums it in a fixed order (every run gives the same
+ * bits), applies Adam to its fp32 master copy and sends the bf16 slice to every
+ * CTA, which puts it into its network.  No cluster barrier, no global-memory
+ * round trip and no host work between steps.  Samples are drawn per epoch through a keyed Feistel
  * permutation of the training set computed on the device.
  *
  * Schedule (ODE_SCHED_LEARNED): predict on the device (mlp_predict: the
@@ -70,8 +70,8 @@ constexpr int LDH = NH + 8;     /* bf16 row stride of hidden-width tiles: 144 B,
 constexpr int W3ROWS = 8;       /* output rows padded to one n8 tile */
 constexpr int TW = 8;           /* warps of a training CTA that compute on samples */
 constexpr int TT = 320;         /* its threads: with two more warps an owner slice of 16 (297 parameters for six
-                                   inputs) takes one round of remote loads and stores instead of two */
-constexpr int TU = 3;           /* rounds at most (40 inputs, 8 CTAs: 865 parameters) */
+                                   inputs) takes one round instead of two */
+constexpr int TU = 3;           /* rounds at most (40 inputs, 8 CTAs: 872 parameters) */
 constexpr int TROWS = 16 * TW;  /* samples per training tile */
 constexpr int PW = 8;           /* warps per prediction block */
 
@@ -316,17 +316,50 @@ struct TrainParams {
   float* master;       /* in: initial fp32 parameters; out (training): trained fp32 parameters (flat layout) */
   __nv_bfloat16* wbf;  /* out (training): bf16 parameters */
   float* grad;         /* out (grad_only): fp32 gradient (flat layout) */
-  float* loss;         /* [2]: summed minibatch losses of the first and the last epoch (atomic adds) */
+  float* loss;         /* [3]: summed minibatch losses of the first and the last epoch (atomic adds); 1 where an
+                          exchange between the CTAs ran into its time limit */
 };
+
+/* The exchange between the CTAs of the cluster: a copy of a piece of this
+ * CTA's shared memory into CTA `q`'s at the same layout, counted by the
+ * receiver's mbarrier (one phase a step: one arrival, by its own thread 0, and
+ * the bytes of every CTA). */
+__device__ __forceinline__ void mbar_init(uint32_t bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n\tfence.mbarrier_init.release.cluster;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar, int bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+/* true when the phase is complete, false after about two seconds */
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, int parity) {
+  const long long t0 = clock64();
+  for (;;) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done) return true;
+    if (clock64() - t0 > 4000000000ll) return false;
+  }
+}
+__device__ __forceinline__ void bulk_to_cta(uint32_t dst, uint32_t src, int bytes, uint32_t bar, int q) {
+  asm volatile(
+      "{\n\t.reg .b32 d, b;\n\tmapa.shared::cluster.u32 d, %0, %4;\n\tmapa.shared::cluster.u32 b, %3, %4;\n\t"
+      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [d], [%1], %2, [b];\n\t}" ::"r"(dst),
+      "r"(src), "r"(bytes), "r"(bar), "r"(q) : "memory");
+}
+/* this thread's stores to shared memory before the copies that read them */
+__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 /* Shared-memory layout of a training CTA (host and device agree on it). */
 struct TrainLayout {
   int ldx, P, S;
-  size_t w1, w2, w3, b1, b2, b3, xs, h1, h2, d1, d2, dout, ys, gp, om, ov, ow, misc, total;
+  size_t w1, w2, w3, b1, b2, b3, xs, h1, h2, d1, d2, dout, ys, gp, rp, lin, ws, om, ov, ow, misc, total;
   __host__ __device__ TrainLayout(int nin, int csize) {
     ldx = kin_steps(nin) * 16 + 8;
     P = NH * nin + NH + NH * NH + NH + NOUT * NH + NOUT;
-    S = (P + csize - 1) / csize;
+    S = ((P + csize - 1) / csize + 7) & ~7; /* 16-byte pieces in fp32 and in bf16 */
     size_t o = 0;
     auto take = [&](size_t bytes) {
       const size_t at = o;
@@ -346,7 +379,10 @@ struct TrainLayout {
     d2 = take((size_t)TROWS * LDH * 2);
     dout = take((size_t)TROWS * 8 * 2);
     ys = take((size_t)TROWS * 2 * 4 * 2);
-    gp = take((size_t)P * 4);
+    gp = take((size_t)csize * S * 4);
+    rp = take((size_t)csize * S * 4);
+    lin = take((size_t)csize * S * 2);
+    ws = take((size_t)S * 2);
     om = take((size_t)S * 4);
     ov = take((size_t)S * 4);
     ow = take((size_t)S * 4);
@@ -355,40 +391,26 @@ struct TrainLayout {
   }
 };
 
-/* Internal parameter order (hidden width NH): W1[NH][nin] b1[NH] W2[NH][NH] b2[NH] W3[2][NH] b3[2].
- * For internal index i: the flat external index for width nh (-1 for a padded
- * unit) and the shared-memory element of the network it lives in. */
-struct ParamSlot {
-  int ext;          /* index in the external layout, or -1 */
-  int kind;         /* 0: bf16 weight (w points into w1/w2/w3), 1: fp32 bias (b) */
-  int off;          /* element offset within the array named by `arr` */
-  int arr;          /* 0 w1, 1 w2, 2 w3, 3 b1, 4 b2, 5 b3 */
-};
-
-__device__ __forceinline__ ParamSlot param_slot(int i, int nin, int nh, int ldx) {
+/* Internal parameter order (hidden width NH): W1[NH][nin] b1[NH] W2[NH][NH] b2[NH] W3[2][NH] b3[2], the
+ * groups of eight in row j of W2 in the order group ^ (j & 7): the rows of a
+ * gradient fragment are stored to distinct banks.
+ * For internal index i the flat external index for width nh, or -1 for a
+ * padded unit. */
+__device__ __forceinline__ int param_ext(int i, int nin, int nh) {
   const Off o(nin, nh);
-  ParamSlot s;
   const int a1 = NH * nin, a2 = a1 + NH, a3 = a2 + NH * NH, a4 = a3 + NH, a5 = a4 + NOUT * NH;
-  if (i < a1) {
-    const int j = i / nin, f = i % nin;
-    s = {j < nh ? o.w1 + j * nin + f : -1, 0, j * ldx + f, 0};
-  } else if (i < a2) {
-    const int j = i - a1;
-    s = {j < nh ? o.b1 + j : -1, 1, j, 3};
-  } else if (i < a3) {
-    const int j = (i - a2) / NH, k = (i - a2) % NH;
-    s = {(j < nh && k < nh) ? o.w2 + j * nh + k : -1, 0, j * LDH + k, 1};
-  } else if (i < a4) {
-    const int j = i - a3;
-    s = {j < nh ? o.b2 + j : -1, 1, j, 4};
-  } else if (i < a5) {
-    const int q = (i - a4) / NH, k = (i - a4) % NH;
-    s = {k < nh ? o.w3 + q * nh + k : -1, 0, q * LDH + k, 2};
-  } else {
-    const int q = i - a5;
-    s = {o.b3 + q, 1, q, 5};
+  if (i < a1) return i / nin < nh ? o.w1 + i : -1;
+  if (i < a2) return i - a1 < nh ? o.b1 + i - a1 : -1;
+  if (i < a3) {
+    const int j = (i - a2) / NH, k = (i - a2) % NH ^ (j & 7) * 8;
+    return j < nh && k < nh ? o.w2 + j * nh + k : -1;
   }
-  return s;
+  if (i < a4) return i - a3 < nh ? o.b2 + i - a3 : -1;
+  if (i < a5) {
+    const int q = (i - a4) / NH, k = (i - a4) % NH;
+    return k < nh ? o.w3 + q * nh + k : -1;
+  }
+  return o.b3 + i - a5;
 }
 
 /* Keyed permutation of [0, n): a 4-round Feistel network on the smallest
@@ -440,17 +462,27 @@ __device__ __forceinline__ uint32_t permute(uint32_t i, const Perm& p) {
 /* One thread-block cluster trains the network for every epoch (see the file
  * comment).  Grid = the cluster: CSIZE CTAs of TT threads.
  *
- * A step is a chain of small dependent products between two cluster barriers,
- * bound by latency (1,920 steps of 1,024 samples, six inputs, 64 of them in each
- * of 16 CTAs; cycles a step: forward and backward 3,400, weight gradients 2,570,
- * the first barrier 1,480, the update 3,490, the second barrier 1,800).  What
- * does not depend on the other CTAs runs between a barrier's arrive and its
- * wait, a tile's first gradient is stored, not added to a zeroed array, and
- * where a parameter lies is worked out once, not every step: 15.1 to 13.1 ms.
- * The two warps without a part in the products gather the next tile into a
- * second buffer while the current one is worked on (its permutation walk and
- * loads, 3,200 cycles, were between the barriers), and one loop over the
- * samples carries all three weight-gradient products: 13.1 to 11.6 ms. */
+ * A step is a chain of small dependent products and two exchanges, bound by
+ * latency.  1,920 steps of 1,024 samples, six inputs, 64 samples in each of 16
+ * CTAs, cycles a step: products 4,930, gradients sent and received 1,310, update
+ * 910, parameters sent and received 1,120, their place in the network 760.
+ * - The exchanges are bulk copies counted by the receiver's mbarrier.  With
+ *   remote loads and stores between cluster barriers they took 6,800 cycles with
+ *   the update (1,200 of them in each barrier's release): 11.6 to 10.7 ms.  One
+ *   thread issues a copy in about 60 cycles, so every warp issues some of the
+ *   16.  Order: a CTA sends its gradient when its products are done and its
+ *   network is not read any more, an owner sends its parameters when it has every
+ *   CTA's gradient, and a CTA goes on when it has every owner's parameters; so
+ *   every buffer has been read before its next copy arrives.
+ * - The rows of W2's gradient fragments go to distinct banks (param_ext; eight
+ *   rows shared a bank): 1,060 cycles of the products; 10.7 to 9.7 ms with the
+ *   spread of the copies.
+ * - Operands that cannot change the update stay out of the slow paths of its
+ *   divisions: 9.7 to 8.7 ms.
+ * - The two warps without a part in the products gather the next tile into a
+ *   second buffer while the current one is worked on, and one loop over the
+ *   samples carries all three weight-gradient products: before these 13.1, after
+ *   them 11.6 ms. */
 template <int KIN, int CSIZE>
 __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
   constexpr int csize = CSIZE;
@@ -476,29 +508,40 @@ __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
   __nv_bfloat16* d2s = (__nv_bfloat16*)(smem + L.d2);
   __nv_bfloat16* douts = (__nv_bfloat16*)(smem + L.dout);
   float* const ys2 = (float*)(smem + L.ys);
-  float* gp = (float*)(smem + L.gp);
+  float* gp = (float*)(smem + L.gp);                         /* this CTA's partial gradient, by owner */
+  float* rp = (float*)(smem + L.rp);                         /* every CTA's partial gradient of the owner slice */
+  __nv_bfloat16* lin = (__nv_bfloat16*)(smem + L.lin);       /* the updated parameters, by owner */
+  __nv_bfloat16* ws = (__nv_bfloat16*)(smem + L.ws);         /* the owner slice's */
   float* om = (float*)(smem + L.om);
   float* ov = (float*)(smem + L.ov);
   float* ow = (float*)(smem + L.ow);
   float* sloss = (float*)(smem + L.misc);
+  const uint32_t bar_g = smem_u32(smem + L.misc + 16), bar_w = bar_g + 8; /* gradients and parameters received */
   const int nh = tp.nh;
   const int lo = rank * L.S, hi = min(L.P, lo + L.S);
   const int ldx = L.ldx;
 
   /* initial network, owner slice, zeroed output-delta padding */
   load_net(net, nin, nh, [&](int i) { return tp.master[i]; });
-  ParamSlot slot[TU]; /* this thread's parameters of the owner slice */
+  int ext[TU]; /* this thread's parameters of the owner slice in the external layout */
 #pragma unroll
   for (int u = 0; u < TU; ++u) {
     const int i = lo + tid + u * TT;
     if (i >= hi) break;
-    slot[u] = param_slot(i, nin, nh, ldx);
-    ow[i - lo] = slot[u].ext >= 0 ? tp.master[slot[u].ext] : 0.f;
+    ext[u] = param_ext(i, nin, nh);
+    ow[i - lo] = ext[u] >= 0 ? tp.master[ext[u]] : 0.f;
     om[i - lo] = 0.f;
     ov[i - lo] = 0.f;
   }
   for (int i = tid; i < TROWS * 8; i += blockDim.x) douts[i] = __float2bfloat16(0.f);
-  if (tid == 0) *sloss = 0.f;
+  for (int i = tid; i < csize * L.S; i += TT) gp[i] = 0.f;
+  for (int i = tid; i < L.S; i += TT) ws[i] = __float2bfloat16(0.f);
+  if (tid == 0) {
+    *sloss = 0.f;
+    mbar_init(bar_g);
+    mbar_init(bar_w);
+  }
+  fence_async_shared();
   cluster.sync();
 
   const float inv_b = 1.f / (float)tp.batch;
@@ -534,12 +577,10 @@ __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
   if (my0 < my1) gather(0, my0, 0, 0);
   __syncthreads();
 
+  bool ok = true;
   for (int step = 0; step < total_steps; ++step) {
     const int epoch = tp.grad_only ? 0 : step / tp.steps_per_epoch;
     const int sie = tp.grad_only ? 0 : step % tp.steps_per_epoch;
-    if (my0 >= my1)
-      for (int i = tid; i < L.P; i += blockDim.x) gp[i] = 0.f;
-
     for (int r0 = my0; r0 < my1; r0 += TROWS) {
       const int valid = min(TROWS, my1 - r0);
       const int kmax = (valid + 15) >> 4;
@@ -637,6 +678,10 @@ __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
          * products of all three, so that their latencies overlap. */
         const bool first = r0 == my0;
         auto put = [&](int i, float v) { gp[i] = first ? v : gp[i] + v; };
+        auto put2 = [&](int i, float v, float w) {
+          float2& to = *reinterpret_cast<float2*>(gp + i);
+          to = first ? make_float2(v, w) : make_float2(to.x + v, to.y + w);
+        };
         const int mt2 = warp >> 1, nb0 = (warp & 1) * 32, mt1 = warp & 3, nt1 = warp >> 2;
         const bool bias2 = (warp & 1) == 0, low = warp < 4;
         const uint32_t ones = g == 0 ? kOnesBf16x2 : 0u;
@@ -671,11 +716,9 @@ __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
         const int gw1 = 0, gb1 = NH * nin, gw2 = gb1 + NH, gb2 = gw2 + NH * NH, gw3 = gb2 + NH, gb3 = gw3 + NOUT * NH;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-          const int j = mt2 * 16 + g, k = nb0 + nt * 8 + 2 * t;
-          put(gw2 + j * NH + k, a2[nt][0]);
-          put(gw2 + j * NH + k + 1, a2[nt][1]);
-          put(gw2 + (j + 8) * NH + k, a2[nt][2]);
-          put(gw2 + (j + 8) * NH + k + 1, a2[nt][3]);
+          const int j = mt2 * 16 + g, k = ((nb0 >> 3) + nt ^ g) * 8 + 2 * t;
+          put2(gw2 + j * NH + k, a2[nt][0], a2[nt][1]);
+          put2(gw2 + (j + 8) * NH + k, a2[nt][2], a2[nt][3]);
         }
         if (bias2 && t == 0) {
           put(gb2 + mt2 * 16 + g, a2b[0]);
@@ -708,68 +751,103 @@ __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
             put(gb3 + 1, a3b[1]);
           }
         }
+        fence_async_shared();
       }
       __syncthreads();
       cur ^= 1;
     }
 
-    /* every CTA's partial gradient is complete and visible cluster-wide after this barrier; meanwhile what
-     * the update needs of this step alone */
-    auto grads = cluster.barrier_arrive();
+    /* every slice of the partial gradient to its owner; meanwhile what the update needs of this step alone */
+    if (lane == 0)
+      for (int q = warp; q < csize; q += TT / 32)
+        bulk_to_cta(smem_u32(rp + rank * L.S), smem_u32(gp + q * L.S), L.S * 4, bar_g, q);
+    if (tid == 0) mbar_expect(bar_g, csize * L.S * 4);
     const int tstep = step + 1;
     const float lr = tp.lr * (epoch < tp.epochs / 2 ? 1.f
                                                      : 0.1f + 0.9f * (float)(tp.epochs - epoch) / (tp.epochs / 2 + 1));
     const float c1 = 1.f - powf(b1, (float)tstep), c2 = 1.f - powf(b2, (float)tstep);
-    cluster.barrier_wait(std::move(grads));
+    ok = __syncthreads_and(mbar_wait(bar_g, step & 1));
+    if (!ok) break;
 #pragma unroll
     for (int u = 0; u < TU; ++u) {
       const int i = lo + tid + u * TT;
       if (i >= hi) break;
-      float part[CSIZE];
-#pragma unroll
-      for (int q = 0; q < CSIZE; ++q) part[q] = cluster.map_shared_rank(gp, q)[i]; /* all loads in flight */
       float gs = 0.f;
 #pragma unroll
-      for (int q = 0; q < CSIZE; ++q) gs += part[q];
-      const ParamSlot& s = slot[u];
+      for (int q = 0; q < CSIZE; ++q) gs += rp[q * L.S + i - lo];
       if (tp.grad_only) {
-        if (s.ext >= 0) tp.grad[s.ext] = gs;
+        if (ext[u] >= 0) tp.grad[ext[u]] = gs;
         continue;
       }
-      if (s.ext < 0) continue; /* padded unit: stays zero */
+      if (ext[u] < 0) continue; /* padded unit: stays zero */
       const int k = i - lo;
       const float mv = b1 * om[k] + (1.f - b1) * gs;
       const float vv = b2 * ov[k] + (1.f - b2) * gs * gs;
       om[k] = mv;
       ov[k] = vv;
-      const float w = ow[k] - lr * (mv / c1) / (sqrtf(vv / c2) + eps);
+      /* Moments of parameters whose gradient has been zero for long decay into the denormals, and one such operand
+       * sends its warp through the slow paths of the divisions and the square root (1,250 cycles a step).  So
+       * operands too small to change the result are replaced: `flat`, sqrt(vv / c2) <= 2.9e-16 (c2 >= 0.000999),
+       * less than half a unit in the last place of eps; `still`, a step of at most 1e-21 (lr <= 1, c1 >= 0.1, the
+       * denominator >= eps), less than a quarter of a unit of the parameter, or zero. */
+      const float w1 = ow[k];
+      const bool flat = vv < 8e-35f;
+      const bool still = lr <= 1.f && ((fabsf(mv) <= 1e-30f && fabsf(w1) > 1e-12f) ||
+                                       (mv == 0.f && __float_as_uint(w1) == 0u));
+      const float den = (flat ? 0.f : sqrtf((flat ? 1.f : vv) / c2)) + eps;
+      const float d = lr * ((still ? 1.f : mv) / c1) / den;
+      const float w = still ? w1 : w1 - d;
       ow[k] = w;
-      const __nv_bfloat16 wb = __float2bfloat16(w);
-      void* base = s.arr == 0 ? (void*)net.w1 : s.arr == 1 ? (void*)net.w2 : s.arr == 2 ? (void*)net.w3
-                 : s.arr == 3 ? (void*)net.b1 : s.arr == 4 ? (void*)net.b2 : (void*)net.b3;
-      if (s.kind == 0) {
-#pragma unroll
-        for (int q = 0; q < CSIZE; ++q) cluster.map_shared_rank((__nv_bfloat16*)base, q)[s.off] = wb;
-      } else {
-#pragma unroll
-        for (int q = 0; q < CSIZE; ++q) cluster.map_shared_rank((float*)base, q)[s.off] = __bfloat162float(wb);
-      }
+      ws[k] = __float2bfloat16(w);
     }
+    fence_async_shared();
     /* loss of the first and the last epoch */
     if (tid == 0 && (tp.grad_only || sie == tp.steps_per_epoch - 1)) {
       if (epoch == 0) atomicAdd(&tp.loss[0], *sloss);
       if (epoch == tp.epochs - 1 || tp.grad_only) atomicAdd(&tp.loss[1], *sloss);
     }
     if (tid == 0 && (tp.grad_only || sie == tp.steps_per_epoch - 1)) *sloss = 0.f;
-    /* the new weights are in place everywhere; the partial gradients may be overwritten */
-    cluster.sync();
+    if (tp.grad_only) break;
+    /* the updated slice to every CTA, which puts the parameters into its network */
+    __syncthreads();
+    if (lane == 0)
+      for (int q = warp; q < csize; q += TT / 32)
+        bulk_to_cta(smem_u32(lin + rank * L.S), smem_u32(ws), L.S * 2, bar_w, q);
+    if (tid == 0) mbar_expect(bar_w, csize * L.S * 2);
+    ok = __syncthreads_and(mbar_wait(bar_w, step & 1));
+    if (!ok) break;
+    const __nv_bfloat16 *l1 = lin, *lb1 = l1 + NH * nin, *l2 = lb1 + NH, *lb2 = l2 + NH * NH, *l3 = lb2 + NH;
+    for (int i = tid; i < NH * NH / 8; i += TT)
+      *reinterpret_cast<uint4*>(net.w2 + (i >> 3) * LDH + (((i >> 3) ^ i) & 7) * 8) =
+          reinterpret_cast<const uint4*>(l2)[i];
+    if (tid < 4 * NH)
+      for (int j = tid >> 2, f = tid & 3; f < nin; f += 4) net.w1[j * ldx + f] = l1[j * nin + f];
+    const int r = tid - (TT - 160); /* the rest over the last 160 threads */
+    if (r >= 0 && r < NH) net.b1[r] = __bfloat162float(lb1[r]);
+    else if (r >= NH && r < 2 * NH) net.b2[r - NH] = __bfloat162float(lb2[r - NH]);
+    else if (r >= 2 * NH && r < 2 * NH + NOUT * NH / 8) {
+      const int i = r - 2 * NH;
+      *reinterpret_cast<uint4*>(net.w3 + (i >> 3) * LDH + (i & 7) * 8) = reinterpret_cast<const uint4*>(l3)[i];
+    } else if (r >= 2 * NH + NOUT * NH / 8 && r < 2 * NH + NOUT * NH / 8 + NOUT) {
+      const int q = r - 2 * NH - NOUT * NH / 8;
+      net.b3[q] = __bfloat162float(l3[NOUT * NH + q]);
+    }
+    __syncthreads();
   }
+  if (!ok) {
+    /* out of time: the host learns of it, and what this CTA has sent has two milliseconds to land */
+    if (tid == 0) tp.loss[2] = 1.f;
+    for (const long long t0 = clock64(); clock64() - t0 < 4000000ll;) {
+    }
+  }
+  /* no CTA leaves while another's copies may still read or write its shared memory */
+  cluster.sync();
   if (!tp.grad_only) {
     for (int i = lo + tid; i < hi; i += blockDim.x) {
-      const ParamSlot s = param_slot(i, nin, nh, ldx);
-      if (s.ext < 0) continue;
-      tp.master[s.ext] = ow[i - lo];
-      tp.wbf[s.ext] = __float2bfloat16(ow[i - lo]);
+      const int e = param_ext(i, nin, nh);
+      if (e < 0) continue;
+      tp.master[e] = ow[i - lo];
+      tp.wbf[e] = __float2bfloat16(ow[i - lo]);
     }
   }
 }
@@ -993,7 +1071,7 @@ static int train(ode_handle* h, Model* m, const std::vector<float>& X, const std
   if (!dX) return rc;
   float* dY = (float*)buf(h, "learn_Y", Y.size() * 4, &rc);
   if (!dY) return rc;
-  float* dL = (float*)buf(h, "learn_loss", 2 * 4, &rc);
+  float* dL = (float*)buf(h, "learn_loss", 3 * 4, &rc);
   if (!dL) return rc;
   cudaStream_t s = h->stream;
   cudaError_t ae;
@@ -1010,7 +1088,7 @@ static int train(ode_handle* h, Model* m, const std::vector<float>& X, const std
   cudaMemcpyAsync(m->d_master, w.data(), np * 4, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(dX, X.data(), X.size() * 4, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(dY, Y.data(), Y.size() * 4, cudaMemcpyHostToDevice, s);
-  cudaMemsetAsync(dL, 0, 2 * 4, s);
+  cudaMemsetAsync(dL, 0, 3 * 4, s);
   TrainParams tp;
   tp.X = dX;
   tp.Y = dY;
@@ -1036,11 +1114,12 @@ static int train(ode_handle* h, Model* m, const std::vector<float>& X, const std
   if (rc != ODE_OK) return rc;
   ee = cudaEventRecord(h->ev1, s);
   if (ee != cudaSuccess) return cuda_fail(h, ee, "event");
-  float l[2] = {0.f, 0.f};
+  float l[3] = {0.f, 0.f, 0.f};
   cudaMemcpyAsync(l, dL, sizeof l, cudaMemcpyDeviceToHost, s);
   cudaError_t e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(h, e, "training");
+  if (l[2] != 0.f) return fail(h, ODE_ECUDA, "training: an exchange between thread blocks ran out of time");
   *loss_first = l[0] / tp.steps_per_epoch;
   *loss_last = l[1] / tp.steps_per_epoch;
   float ms = 0.f;
@@ -1268,14 +1347,14 @@ int ode_learn_gradcheck(ode_handle* h, int nin, int nh, int64_t batch, const flo
   if (!dG) return rc;
   float* dP = (float*)buf(h, "gc_P", np * 4, &rc);
   if (!dP) return rc;
-  float* dL = (float*)buf(h, "gc_L", 2 * 4, &rc);
+  float* dL = (float*)buf(h, "gc_L", 3 * 4, &rc);
   if (!dL) return rc;
   cudaStream_t s = h->stream;
   cudaMemcpyAsync(dX, x, (size_t)batch * nin * 4, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(dY, y, (size_t)batch * NOUT * 4, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(dP, params, np * 4, cudaMemcpyHostToDevice, s);
   cudaMemsetAsync(dG, 0, np * 4, s);
-  cudaMemsetAsync(dL, 0, 2 * 4, s);
+  cudaMemsetAsync(dL, 0, 3 * 4, s);
   TrainParams tp;
   std::memset(&tp, 0, sizeof tp);
   tp.X = dX;
@@ -1292,12 +1371,13 @@ int ode_learn_gradcheck(ode_handle* h, int nin, int nh, int64_t batch, const flo
   tp.loss = dL;
   rc = launch_train(h, tp, s, nullptr);
   if (rc != ODE_OK) return rc;
-  float l[2];
+  float l[3];
   cudaMemcpyAsync(grad, dG, np * 4, cudaMemcpyDeviceToHost, s);
   cudaMemcpyAsync(l, dL, sizeof l, cudaMemcpyDeviceToHost, s);
   cudaError_t e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(h, e, "gradcheck");
+  if (l[2] != 0.f) return fail(h, ODE_ECUDA, "gradcheck: an exchange between thread blocks ran out of time");
   *loss = l[0];
   return ODE_OK;
 }
