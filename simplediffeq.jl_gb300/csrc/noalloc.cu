@@ -52,7 +52,7 @@ static_assert(kScratchBytes == 33024, "scratch size stated in the header comment
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 typedef gbode::RhsLorenz<double, double> LorenzFP64;
-GBODE_ENTRY(gbode_noalloc_atsit5_persistent_lorenz3_fp64, persistent, gbode::MTsit5, gbode::PFP64, LorenzFP64)
+GBODE_ENTRY(gbode_noalloc_atsit5_persistent_lorenz3_fp64, unstaged, gbode::MTsit5, gbode::PFP64, LorenzFP64)
 
 /* the attempt cap used when the caller gives none (the same as ode_ensemble_solve) */
 constexpr long long kDefaultMaxIters = 1000000;

@@ -654,8 +654,8 @@ int plain_block(int64_t n, int nsm, int maxb) {
   return best;
 }
 
-/* Most blocks a persistent launch in FP64 should take for the SM
- * sub-partitions to hold the same number of warps.  For a few more warps than
+/* Most blocks a persistent launch should take.  In FP64 for the SM
+ * sub-partitions to hold the same number of warps: for a few more warps than
  * there are sub-partitions some hold two, which share the FP64 pipe and end
  * last, while the others wait; with one warp on each the lanes that finish
  * first take the remaining trajectories.  Up to 1.4 warps a sub-partition
@@ -665,10 +665,18 @@ int plain_block(int64_t n, int nsm, int maxb) {
  * Pol with saveat, AVern9 three-body: 20,000 trajectories 1.41, 1.16, 1.19,
  * 1.10, 1.25; 25,000 (the first three) 1.26, 1.05, 1.16; 32,000 1.06, 0.95,
  * 1.05, 1.02, 1.13; 38,900 (the first three) 0.92, 0.84, 0.95.  Single
- * precision gains nothing from it. */
+ * precision gains nothing from it.
+ *
+ * Verner 9 without saveat has registers for more warps than its lanes gain
+ * from: with two warps a sub-partition in FP64 and three in single precision,
+ * against three and five, fewer trajectories share the pipe with the longest
+ * one.  Restricted three-body problem, 150,000 in FP64 61.0 against 65.3 ms,
+ * 131,072 in FP32 with compensation 3.6 against 3.8 ms. */
 int64_t even_blocks(const ode_handle* h, const ode_solve_args* a, int block) {
   const int64_t warps = (a->n + 31) / 32, slots = (int64_t)h->nsm * 4;
-  if (a->precision != ODE_FP64 || warps <= slots || warps * 10 > slots * 14 || block > 128) return INT64_MAX;
+  const int64_t most = a->alg == ODE_ALG_AVERN9 && a->nsave == 0 && block <= 128
+                           ? slots * (a->precision == ODE_FP64 ? 2 : 3) / (block / 32) : INT64_MAX;
+  if (a->precision != ODE_FP64 || warps <= slots || warps * 10 > slots * 14 || block > 128) return most;
   return slots / (block / 32);
 }
 
