@@ -373,12 +373,18 @@ int small_ring_bytes(const ode_solve_args* a) { return (36 * stage_unit_bytes(a)
  * fewer warps, which the integer pipe's latency needs; time of the register
  * kernel over the crowded one's on Van der Pol, 0 / 20 / 200 save points:
  * 50,000 trajectories 1.32 / 1.06 / 0.95, 100,000 1.26 / 1.07 / 1.02, 200,003
- * 1.23 / 1.10 / 1.05.  Verner 9 on the three-body problem: 0.95 to 1.05. */
-bool crowded(const ode_handle* h, const ode_solve_args* a) {
+ * 1.23 / 1.10 / 1.05.  Plain schedule, where a lane interpolates its save points
+ * alone from stages in shared memory, 0 / 20 / 50 / 100 / 200: 60,000 0.95 with
+ * none, 120,000 1.12 / 1.41 / 1.28 / 1.22 / 0.98, 400,000 1.13 / 1.38 / 1.26 /
+ * 1.18 / 0.95; so five warps, and no more than 100 save points.  Verner 9 on the
+ * three-body problem: 0.95 to 1.05. */
+bool crowded(const ode_handle* h, const ode_solve_args* a, int sched) {
   if ((a->alg != ODE_ALG_ATSIT5 && a->alg != ODE_ALG_AVERN7) || a->precision != ODE_FP64 ||
       a->controller == ODE_CTRL_REF)
     return false;
-  return ensemble_size(h, a) > (int64_t)h->nsm * 4 * (a->alg == ODE_ALG_AVERN7 && a->nsave > 0 ? 160 : 64);
+  const bool v7 = a->alg == ODE_ALG_AVERN7, plain = sched == ODE_SCHED_PLAIN;
+  if (v7 && plain && a->nsave > 100) return false;
+  return ensemble_size(h, a) > (int64_t)h->nsm * 4 * (v7 && (plain || a->nsave > 0) ? 160 : 64);
 }
 
 /* Whether its kernel keeps the stages in shared memory and forms their linear
@@ -398,7 +404,7 @@ bool crowded(const ode_handle* h, const ode_solve_args* a) {
  * latency shows (the Lorenz solve above at 8: no gain). */
 bool use_integer_pipe(const ode_handle* h, const ode_solve_args* a, int sched) {
   const bool staged = !std::strcmp(entry_kind(a->alg, sched, a->nsave), "staged");
-  return crowded(h, a) && stage_slice_bytes(a) + (staged ? small_ring_bytes(a) : 0) <= 19456;
+  return crowded(h, a, sched) && stage_slice_bytes(a) + (staged ? small_ring_bytes(a) : 0) <= 19456;
 }
 
 /* Launch shape of an untuned run-time compiled kernel: 128 threads and 12 KB
@@ -454,7 +460,7 @@ std::string kernel_key(ode_handle* h, const ode_solve_args* a, int sched) {
   char b[160];
   snprintf(b, sizeof b, "%s|%s|%d|%d|%s|%d%s%s%s", alg_name(a->alg), kernel_kind(h, a, sched), a->rhs, a->dim,
            prec_name(a->precision), a->output >= ODE_OUTPUT_USER ? a->output : 0, h->bounds_check ? "|chk" : "",
-           ctrl_suffix(ctrl_variant(a)), crowded(h, a) ? "|crowded" : "");
+           ctrl_suffix(ctrl_variant(a)), crowded(h, a, sched) ? "|crowded" : "");
   return b;
 }
 
@@ -462,7 +468,7 @@ std::string kernel_key(ode_handle* h, const ode_solve_args* a, int sched) {
  * dim, schedule kind). */
 std::string jit_source(ode_handle* h, const ode_solve_args* a, int sched) {
   std::string src;
-  if (crowded(h, a)) src += "#define GBODE_CROWDED 1\n";
+  if (crowded(h, a, sched)) src += "#define GBODE_CROWDED 1\n";
   if (ctrl_variant(a) == ODE_CTRL_FP64) src += "#define GBODE_CTRL64 1\n";
   if (ctrl_variant(a) == ODE_CTRL_DS) src += "#define GBODE_CTRL_DS 1\n";
   if (ctrl_variant(a) == ODE_CTRL_REF) src += "#define GBODE_REF 1\n";
@@ -599,7 +605,7 @@ int get_kernel(ode_handle* h, const ode_solve_args* a, int sched, CUfunction* fn
     return ODE_OK;
   }
   const char* kind = kernel_kind(h, a, sched);
-  const bool crowd = crowded(h, a);
+  const bool crowd = crowded(h, a, sched);
   for (const AotEntry& e : kAotEntries) {
     if (!h->bounds_check && ctrl_variant(a) == ODE_CTRL_DS && a->output < ODE_OUTPUT_USER && e.alg == a->alg &&
         e.rhs == a->rhs &&
@@ -1151,7 +1157,7 @@ int solve_impl(ode_handle* h, const ode_solve_args* a, ode_solve_out* o, ode_sol
   /* the place where the persistent kernels' warps park trajectories to merge (Feed in ode_solver.cuh) */
   int* park_ctl = nullptr;
   size_t park_bytes = 0;
-  if (sched != ODE_SCHED_PLAIN && crowded(h, a)) {
+  if (sched != ODE_SCHED_PLAIN && crowded(h, a, sched)) {
     const size_t cap = (size_t)gridx * block;
     park_bytes = (PARK_FLAGS + cap) * sizeof(int);
     if (!(park_ctl = (int*)buf(h, nm("park_ctl"), park_bytes, &rc))) return rc;
