@@ -2809,7 +2809,9 @@ __device__ __forceinline__ void run_adaptive_staged_or_persistent(const KParams&
  * registers in FP32 with compensation, 238 to 154 in FP64, and the restricted
  * three-body problem's long lone trajectories, which wait on instruction
  * fetch, 3 to 5% and 1% faster (16,384 in FP32, tolerance 1e-6: 2.43 to 2.33 ms).
- * For the smaller methods the registers that go free bring more resident warps
+ * So do the crowded kernels: 1,000,000 Lorenz 68.8 to 60.4 ms, 65,536 7.0 to
+ * 6.6, 400,000 Van der Pol with Verner 7 22.7 to 21.8.
+ * For the smaller methods otherwise the registers that go free bring more resident warps
  * than there are trajectories to refill them with: Verner 7 in FP32, 400,000
  * Van der Pol 0.77 to 0.90 ms. */
 template <class M, class PR, int D, class F, bool SAVES>
@@ -3326,7 +3328,7 @@ __device__ __forceinline__ void run_onestep(const KParams& P) {
 #define GBODE_ENTRY_persistent(NAME, M, PR, RHS)                                             \
   extern "C" __global__ void __launch_bounds__(GBODE_BLOCK) NAME(gbode::KParams P) {                \
     gbode::run_adaptive_unstaged<M<PR, RHS::D, RHS>, PR, RHS::D, RHS,                       \
-                                 (M<PR, RHS::D, RHS>::NK < 16)>(P);                         \
+                                 (M<PR, RHS::D, RHS>::NK < 16 && !gbode::CROWDED)>(P);      \
   }
 #define GBODE_ENTRY_unstaged(NAME, M, PR, RHS)                                               \
   extern "C" __global__ void __launch_bounds__(GBODE_BLOCK) NAME(gbode::KParams P) {                \
