@@ -1180,8 +1180,10 @@ int ode_learn_fit(ode_handle* h, const ode_solve_args* a, const ode_learn_opts* 
   if (rc != ODE_OK && rc != ODE_ETRAJ) return rc;
   const auto t1 = std::chrono::steady_clock::now();
 
-  Model* m = h->model ? h->model : new Model();
-  h->model = m;
+  /* a fit works on the spare model, which takes the fitted one's place when
+   * all has succeeded: a fit that fails leaves the fitted model as it was */
+  Model* m = h->spare_model ? h->spare_model : new Model();
+  h->spare_model = m;
   const int nin = a->nparams + a->dim;
   if (m->nin != nin || m->nh != o.hidden) {
     if (m->d_master) cudaFree(m->d_master);
@@ -1264,6 +1266,7 @@ int ode_learn_fit(ode_handle* h, const ode_solve_args* a, const ode_learn_opts* 
   int ctas = 0;
   rc = train(h, m, Xs, Ys, nb, o, &lf, &ll, &kms, &ctas);
   if (rc != ODE_OK) return rc;
+  std::swap(h->model, h->spare_model);
   const auto t2 = std::chrono::steady_clock::now();
   if (rep) {
     rep->loss_first = lf;

@@ -851,7 +851,8 @@ void ode_destroy(ode_handle* h) {
   for (auto& kv : h->bufs)
     if (kv.second.ptr) cudaFree(kv.second.ptr);
   for (CUmodule m : h->modules) g_drv.cuModuleUnload(m);
-  if (h->model) model_free(h->model);
+  model_free(h->model);
+  model_free(h->spare_model);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->stream) cudaStreamDestroy(h->stream);

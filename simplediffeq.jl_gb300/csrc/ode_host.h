@@ -81,7 +81,8 @@ struct ode_handle {
   std::map<std::string, CUfunction> sde_kernels;
   std::vector<gbode::GraphEntry> graphs;
   unsigned long long graph_tick = 0;
-  gbode::Model* model = nullptr;
+  gbode::Model* model = nullptr;        /* the fitted cost model */
+  gbode::Model* spare_model = nullptr;  /* what a fit works on (ode_learn_fit) */
   bool bounds_check = false;  /* ode_set_bounds_check */
   int64_t tune_n = 0;         /* while autotuning: the whole ensemble's size */
 };
