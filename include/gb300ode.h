@@ -443,6 +443,12 @@ int ode_learn_predict(ode_handle* h, const ode_solve_args* a, float* log_attempt
  * mean_b sum_o (out - y)^2 and the loss. */
 int ode_learn_gradcheck(ode_handle* h, int nin, int nh, int64_t batch, const float* params, const float* x,
                         const float* y, float* grad, float* loss);
+/* Clock cycles that an exchange between the training kernel's thread blocks
+ * may take before ode_learn_fit and ode_learn_gradcheck return ODE_ECUDA (0:
+ * the default, 4e9; below 0: none, every exchange fails at once, for
+ * verification).  The context stays usable, and the handle keeps the model
+ * fitted before. */
+int ode_learn_set_wait_limit(ode_handle* h, int64_t cycles);
 
 /* ---- allocation-free solve ------------------------------------------------
  * No counterpart in the reference: an entry point for callers that cannot

@@ -155,6 +155,7 @@ def load():
     lib.ode_learn_predict.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveArgs), ctypes.c_void_p, ctypes.c_void_p]
     lib.ode_learn_gradcheck.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int64, ctypes.c_void_p,
                                         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    lib.ode_learn_set_wait_limit.argtypes = [ctypes.c_void_p, ctypes.c_int64]
     lib.ode_autotune.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveArgs), ctypes.c_int64, ctypes.POINTER(TuneReport)]
     lib.ode_tune_save.argtypes = [ctypes.c_void_p, ctypes.c_char_p]
     lib.ode_tune_load.argtypes = [ctypes.c_void_p, ctypes.c_char_p]
@@ -285,6 +286,9 @@ class Handle:
         self.check(self.lib.ode_learn_gradcheck(self.h, nin, nh, x.shape[0], params.ctypes.data, x.ctypes.data,
                                                 y.ctypes.data, grad.ctypes.data, loss.ctypes.data))
         return grad, float(loss[0])
+
+    def learn_set_wait_limit(self, cycles):
+        self.check(self.lib.ode_learn_set_wait_limit(self.h, int(cycles)))
 
     def learn_predict(self, args, n):
         la = np.zeros(n, dtype=np.float32)
