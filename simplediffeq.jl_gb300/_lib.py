@@ -28,7 +28,7 @@ RET_DEFAULT, RET_DTMIN, RET_MAXITERS, RET_NAN = 0, 1, 2, 3
 # Every symbol include/gb300ode.h declares.
 EXPORTS = ["ode_abi_version", "ode_create", "ode_destroy", "ode_last_error", "ode_ensemble_solve",
            "ode_fixed_grid", "ode_rhs_compile", "ode_output_compile", "ode_learn_default_opts", "ode_learn_fit",
-           "ode_learn_predict", "ode_learn_gradcheck", "ode_ensemble_solve_noalloc", "ode_autotune",
+           "ode_learn_predict", "ode_learn_gradcheck", "ode_learn_set_wait_limit", "ode_ensemble_solve_noalloc", "ode_autotune",
            "ode_ensemble_solve_everystep", "ode_sde_solve", "ode_sde_compile", "ode_sde_compile_noise",
            "ode_set_bounds_check", "ode_tune_save", "ode_tune_load", "ode_rhs_builtin"]
 SDE = {"gbm": 0, "ou": 1, "lorenz": 2, "mult": 3}
