@@ -2192,6 +2192,19 @@ __device__ __forceinline__ void lane_unpark(const KParams& P, Lane<PR, D, F, NK,
   rhs_loaded(l.f);
 }
 
+/* An entry's flag: set by the lane that has parked the trajectory, seen by a
+ * lane of the warp that takes it up.  Release and acquire, with a __syncwarp
+ * from the lane that sees the flag to the one that reads the entry: the order
+ * that fences between plain accesses do not give. */
+__device__ __forceinline__ void flag_set(int* flag) {
+  asm volatile("st.release.gpu.s32 [%0], 1;" ::"l"(flag) : "memory");
+}
+__device__ __forceinline__ int flag_seen(const int* flag) {
+  int v;
+  asm volatile("ld.acquire.gpu.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+  return v;
+}
+
 /* Hands a warp's lanes their trajectories.  While the device counter has
  * positions left, a lane that finished takes the next one (one atomicAdd per
  * warp for all lanes that need work), mapped through P.order.
@@ -2289,7 +2302,7 @@ struct Feed {
     if (tail > head && idle > 0) {
       const int most = tail - head < idle ? tail - head : idle;
       int there = 0;
-      if (lane < most) there = __ldcg(ctl + PARK_FLAGS + head + lane);
+      if (lane < most) there = flag_seen(ctl + PARK_FLAGS + head + lane);
       const unsigned ready = __ballot_sync(FULL, there != 0);
       const int take = ready == FULL ? 32 : __ffs(~ready) - 1;
       int got = 0;
@@ -2298,7 +2311,7 @@ struct Feed {
         got = __shfl_sync(FULL, got, 0);
       }
       if (got) {
-        __threadfence();
+        __syncwarp();
         const int rank = __popc(~act & ((1u << lane) - 1u));
         if (!active && rank < take) {
           lane_unpark<PR, D, F, NK, KS, M::FSAL != 0>(P, l, head + rank);
@@ -2320,8 +2333,7 @@ struct Feed {
         const int i = base + __popc(act & ((1u << lane) - 1u));
         if (active) {
           lane_park<PR, D, F, NK, KS, M::FSAL != 0>(P, l, i);
-          __threadfence();
-          __stcg(ctl + PARK_FLAGS + i, 1);
+          flag_set(ctl + PARK_FLAGS + i);
           active = false;
           exhausted = true;
         }
