@@ -1305,8 +1305,9 @@ template <class R, int D, int STRIDE>
 struct StageRows {
   R* p;
   /* whether a linear combination of the last attempt was not decided on the
-   * integer pipe; attempts left that do without it */
-  bool missed;
+   * integer pipe; attempts left that do without it; whether the warp does
+   * without it this time */
+  bool missed, off;
   int rest;
   __device__ __forceinline__ StageRow<R, STRIDE> operator[](int q) const { return StageRow<R, STRIDE>{p + q * D * STRIDE}; }
 };
@@ -1410,9 +1411,9 @@ struct MInt : M {
                                                  bool want_err) {
     const R h = (R)dt;
     /* A row with a zero stage is never decided on the integer pipe.  Where
-     * that keeps happening (a component at rest), the lane, and with it the
-     * lanes it runs with, does without it for the next attempts. */
-    const bool on_int = !__any_sync(__activemask(), k.rest > 0);
+     * that keeps happening (a component at rest), the lane, and with it its
+     * warp (StageTypes::vote), does without it for the next attempts. */
+    const bool on_int = !k.off;
     bool missed = false;
     R tmp[D], du[D];
     IcSpan E[D];
@@ -1508,6 +1509,7 @@ template <bool SHARED, class M, class PR, int D, class F> struct StageTypes {
   typedef typename PR::R KS[M::NK][D];
   enum { SLICE = 1 };
   __device__ static __forceinline__ void bind(KS&, typename PR::R*) {}
+  __device__ static __forceinline__ void vote(KS&, bool) {}
 };
 template <class M, class PR, int D, class F> struct StageTypes<true, M, PR, D, F> {
   typedef MInt<M, PR, D, F> Method;
@@ -1516,7 +1518,12 @@ template <class M, class PR, int D, class F> struct StageTypes<true, M, PR, D, F
   __device__ static __forceinline__ void bind(KS& k, typename PR::R* slice) {
     k.p = slice + (threadIdx.x & 31);
     k.missed = false;
+    k.off = false;
     k.rest = 0;
+  }
+  /* by all lanes of a warp before an attempt, active ones or not */
+  __device__ static __forceinline__ void vote(KS& k, bool active) {
+    k.off = __any_sync(0xffffffffu, active && k.rest > 0);
   }
 };
 
@@ -2108,9 +2115,16 @@ __device__ __forceinline__ void run_adaptive_plain(const KParams& P) {
   typedef typename ST::Method MM;
   __shared__ typename PR::R kmem[kWarpsPerBlock][ST::SLICE];
   Totals tot = {0, 0, 0};
-  if (i < P.n) {
-    Lane<PR, D, F, M::NK, typename ST::KS> l;
-    ST::bind(l.k, kmem[threadIdx.x >> 5]);
+  Lane<PR, D, F, M::NK, typename ST::KS> l;
+  ST::bind(l.k, kmem[threadIdx.x >> 5]);
+  if constexpr (Stages<M, PR, D, F, 0>::SHARED) {
+    /* all lanes of a warp together, for the vote */
+    bool active = i < P.n && !adaptive_start<MM>(P, i, l, tot);
+    while (__any_sync(0xffffffffu, active)) {
+      ST::vote(l.k, active);
+      if (active) active = !adaptive_iter<MM, true>(P, l, tot);
+    }
+  } else if (i < P.n) {
     if (!adaptive_start<MM>(P, i, l, tot)) {
       while (!adaptive_iter<MM, true>(P, l, tot)) {
       }
@@ -2401,6 +2415,7 @@ __device__ __forceinline__ void run_adaptive_persistent(const KParams& P, typena
   for (;;) {
     if (!feed.next<MM>(P, l, active, tot)) break;
     if (!__any_sync(FULL, active)) continue;
+    ST::vote(l.k, active);
     if (active && adaptive_iter<MM, SAVES>(P, l, tot)) active = false;
   }
   flush_totals(P, tot);
@@ -2505,6 +2520,7 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P, typename P
   for (;;) {
     if (!feed.next<MM>(P, l, active, tot)) break;
     if (!__any_sync(FULL, active)) continue;
+    ST::vote(l.k, active);
     R nh[D], nc[D];
     Accepted<T> st;
     int r = TRY_REJECTED, njobs = 0;
@@ -2707,6 +2723,7 @@ __device__ __forceinline__ void run_adaptive_staged2(const KParams& P, typename 
   for (;;) {
     if (!feed.next<MM>(P, l, active, tot)) break;
     if (!__any_sync(FULL, active)) continue;
+    ST::vote(l.k, active);
     R nh[D], nc[D];
     Accepted<T> st;
     int r = TRY_REJECTED, njobs = 0;

@@ -23,3 +23,9 @@ def test_parking_flags_are_released_and_acquired():
     assert re.search(r"flag_seen\(const int\* flag\) \{\s*int v;\s*asm volatile\(\"ld\.acquire\.gpu\.", src)
     taken = src[src.index("flag_seen(ctl"):src.index("lane_unpark<PR, D, F, NK, KS, M::FSAL")]
     assert "__syncwarp()" in taken
+
+
+def test_no_vote_over_the_threads_that_happen_to_be_there():
+    """__activemask() names threads that nothing makes take part in the vote that follows it."""
+    for path in glob.glob(os.path.join(CSRC, "*.cu*")) + glob.glob(os.path.join(CSRC, "*.h")):
+        assert "__activemask" not in code(os.path.basename(path)), path
