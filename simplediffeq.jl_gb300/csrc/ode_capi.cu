@@ -300,7 +300,6 @@ bool use_adaptive_split(const ode_handle* h, const ode_solve_args* a, int sched)
   const bool separable = a->rhs == ODE_RHS_LORENZ || a->rhs == ODE_RHS_VANDERPOL || a->rhs == ODE_RHS_LINEAR;
   return a->alg == ODE_ALG_ATSIT5 && sched != ODE_SCHED_PLAIN && separable && a->output == ODE_OUTPUT_STATE &&
          a->precision == ODE_FP64 && a->controller != ODE_CTRL_REF && a->dim >= 2 && a->dim <= 8 &&
-         !h->bounds_check &&
          (ensemble_size(h, a) + 31) / 32 <= (int64_t)(a->dim <= 4 ? h->nsm * (4 / a->dim) : h->nsm * 4 / a->dim);
 }
 
@@ -1298,7 +1297,7 @@ int solve_impl(ode_handle* h, const ode_solve_args* a, ode_solve_out* o, ode_sol
     if (hchk[0] || bad >= 0) {
       char m[256];
       snprintf(m, sizeof m, "bounds check: violation bits 0x%x (1 trajectory, 2 save point, 4 every-step row, "
-               "8 staging ring, 16 order); trajectory %lld started %u times",
+               "8 staging ring, 16 order, 32 parking place); trajectory %lld started %u times",
                hchk[0], (long long)bad, bad >= 0 ? hchk[16 + (size_t)bad] : 1u);
       return fail(h, ODE_ECHECK, m);
     }

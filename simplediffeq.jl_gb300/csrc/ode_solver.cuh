@@ -74,7 +74,7 @@ namespace gbode {
  * the access is skipped (or clamped to a valid index).  Each trajectory start
  * is counted in P.visited, so the host can verify that the schedule handed
  * every trajectory out exactly once.  Without the flag the checks vanish. */
-enum { CHK_TRAJ = 1, CHK_SAVE = 2, CHK_STEP = 4, CHK_RING = 8, CHK_ORDER = 16 };
+enum { CHK_TRAJ = 1, CHK_SAVE = 2, CHK_STEP = 4, CHK_RING = 8, CHK_ORDER = 16, CHK_PARK = 32 };
 #ifdef GBODE_BOUNDS_CHECK
 #define GBODE_CHECK(P, cond, bit) ((cond) ? true : (atomicOr((P).check_flags, (unsigned)(bit)), false))
 #else
@@ -1636,7 +1636,7 @@ template <class PR, int D, class F, int NK, class KS>
 __device__ __forceinline__ void lane_load(const KParams& P, long long idx, Lane<PR, D, F, NK, KS>& l) {
   if (!GBODE_CHECK(P, idx >= 0 && idx < P.n, CHK_TRAJ)) idx = 0;
 #ifdef GBODE_BOUNDS_CHECK
-  atomicAdd(&P.visited[idx], 1u);
+  if (P.visited) atomicAdd(&P.visited[idx], 1u);
 #endif
   typedef typename PR::R R;
   typedef typename PR::T T;
@@ -2327,7 +2327,7 @@ struct Feed {
       if (got) {
         __syncwarp();
         const int rank = __popc(~act & ((1u << lane) - 1u));
-        if (!active && rank < take) {
+        if (!active && rank < take && GBODE_CHECK(P, head >= 0 && head + rank < P.park_cap, CHK_PARK)) {
           lane_unpark<PR, D, F, NK, KS, M::FSAL != 0>(P, l, head + rank);
           active = true;
         }
@@ -2345,7 +2345,7 @@ struct Feed {
       base = __shfl_sync(FULL, base, 0);
       if (room) {
         const int i = base + __popc(act & ((1u << lane) - 1u));
-        if (active) {
+        if (active && GBODE_CHECK(P, i >= 0 && i < P.park_cap, CHK_PARK)) {
           lane_park<PR, D, F, NK, KS, M::FSAL != 0>(P, l, i);
           flag_set(ctl + PARK_FLAGS + i);
           active = false;
@@ -3081,6 +3081,7 @@ struct AdaptiveSplitTsit5 {
       P.ev_t = 0;
       P.stats = 0;
       P.us = 0;
+      P.visited = 0;
     }
     const int lane = threadIdx.x & 31;
     const long long i = (long long)blockIdx.x * 32 + lane;
@@ -3099,6 +3100,7 @@ struct AdaptiveSplitTsit5 {
       Q.u_final = 0;
       Q.ev_t = 0;
       Q.us = 0;
+      Q.visited = 0;
       lane_load(Q, 0, l);
     }
     l.k.k[0][0] = FS::template rhs<C>(l.f, l.uh, l.t);
