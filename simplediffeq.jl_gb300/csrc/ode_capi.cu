@@ -1752,9 +1752,13 @@ int ode_autotune(ode_handle* h, const ode_solve_args* a, int64_t sample, ode_tun
   /* large jobs (Kuramoto-12: 804 bytes) also try the smallest ring that holds
    * one round, which leaves room for the most warps per SM */
   const int fit = (32 * job + 511) / 512 * 512;
-  for (int block : {128, 64, 32}) {
+  /* the component split has one block size and no ring */
+  const bool split = use_adaptive_split(h, &ta, ta.schedule);
+  for (int block : split ? std::vector<int>{32 * D} : std::vector<int>{128, 64, 32}) {
     std::vector<int> rings;
-    if (staged) {
+    if (split) {
+      rings.push_back(0);
+    } else if (staged) {
       if ((ic || fit > 12288) && fit / 32 * block <= 49152) rings.push_back(fit);
       for (int ring : {12288, 16384, 24576, 36864, 49152})
         if (ring / 32 * block <= 49152 && ring / job >= 32) rings.push_back(ring);
@@ -1813,9 +1817,9 @@ int ode_autotune(ode_handle* h, const ode_solve_args* a, int64_t sample, ode_tun
                                    : std::vector<int>{0, 0, 0};  /* 0: the default kernel won */
   if (rep) {
     rep->variants = tried;
-    rep->block = best >= 0 ? vars[best].block : block_of(h, fn0);
+    rep->block = best >= 0 ? vars[best].block : split ? 32 * D : block_of(h, fn0);
     rep->max_registers = best >= 0 ? vars[best].regs : 0;
-    rep->stage_bytes = best >= 0 ? vars[best].stage : stage_of(h, fn0);
+    rep->stage_bytes = best >= 0 ? vars[best].stage : split ? 0 : stage_of(h, fn0);
     rep->default_ms = base_ms;
     rep->best_ms = best_ms;
     rep->sample = m;
