@@ -16,8 +16,8 @@ enum { RET_DEFAULT = 0, RET_DTMIN = 1, RET_MAXITERS = 2, RET_NAN = 3 };
  * flag per entry that its trajectory is there. */
 enum { PARK_IDLE = 0, PARK_WARPS = 1, PARK_TAIL = 2, PARK_HEAD = 3, PARK_SLOTS = 16, PARK_MAX_SLOTS = 1024,
        PARK_FLAGS = PARK_SLOTS + PARK_MAX_SLOTS };
-/* doubles of a parked trajectory of dimension D: at most three per component and 12 */
-constexpr int park_words(int D) { return 3 * D + 12; }
+/* doubles of a parked trajectory of dimension D: at most two per component and 10 */
+constexpr int park_words(int D) { return 2 * D + 10; }
 
 struct KParams {
   long long n;             /* trajectories */
@@ -50,8 +50,8 @@ struct KParams {
   const int* order;        /* persistent: position -> trajectory, or 0 for identity */
   unsigned long long* counter;   /* persistent: next position to hand out (zeroed before launch) */
   int* park_ctl;           /* persistent: the parking place's words (ParkWord, then the sub-partitions' warp
-                              counts and the entries' flags; zeroed before launch), or 0: no parking */
-  double* park;            /* [PARK_WORDS][park_cap] parked trajectories */
+                              counts and the entries' flags; zeroed before launch), or 0: not a crowded kernel */
+  double* park;            /* [park_words(dim)][park_cap] parked trajectories */
   long long park_cap;      /* entries: the launch's lanes */
   int park_min, park_slots; /* warps below which none parks; SM sub-partitions */
   unsigned long long* stats;     /* [2] attempts and saves summed over trajectories, or 0 */

@@ -2135,7 +2135,9 @@ __device__ __forceinline__ void run_adaptive_plain(const KParams& P) {
 
 /* ------------------------------------------------------------------ work for the persistent schedules */
 /* A trajectory between two attempts, to and from entry i of the parking place
- * (past L1: another SM reads it).  Parameters are loaded again. */
+ * (past L1: another SM reads it).  Parameters are loaded again.  Only the
+ * crowded kernels do this: FP64, no compensation, not the reference's
+ * arithmetic. */
 template <class PR, int D, class F, int NK, class KS, bool FSAL>
 __device__ __forceinline__ void lane_park(const KParams& P, Lane<PR, D, F, NK, KS>& l, long long i) {
   double* e = P.park + i;
@@ -2143,7 +2145,6 @@ __device__ __forceinline__ void lane_park(const KParams& P, Lane<PR, D, F, NK, K
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     __stcg(e, (double)l.uh[d]); e += c;
-    if (PR::KAHAN) { __stcg(e, (double)l.uc[d]); e += c; }
     if (FSAL) { __stcg(e, (double)l.k[0][d]); e += c; }
   }
   __stcg(e, (double)l.t); e += c;
@@ -2161,9 +2162,6 @@ __device__ __forceinline__ void lane_park(const KParams& P, Lane<PR, D, F, NK, K
 #ifdef GBODE_CTRL64
   __stcg(e, l.lqold); e += c;
 #endif
-#ifdef GBODE_REF
-  __stcg(e, l.qold); e += c;
-#endif
 }
 template <class PR, int D, class F, int NK, class KS, bool FSAL>
 __device__ __forceinline__ void lane_unpark(const KParams& P, Lane<PR, D, F, NK, KS>& l, long long i) {
@@ -2175,7 +2173,6 @@ __device__ __forceinline__ void lane_unpark(const KParams& P, Lane<PR, D, F, NK,
   for (int d = 0; d < D; ++d) {
     l.uh[d] = (R)__ldcg(e); e += c;
     l.uc[d] = (R)0;
-    if (PR::KAHAN) { l.uc[d] = (R)__ldcg(e); e += c; }
     if (FSAL) { l.k[0][d] = (R)__ldcg(e); e += c; }
   }
   l.t = (T)__ldcg(e); e += c;
@@ -2197,9 +2194,6 @@ __device__ __forceinline__ void lane_unpark(const KParams& P, Lane<PR, D, F, NK,
 #endif
 #ifdef GBODE_CTRL64
   l.lqold = __ldcg(e); e += c;
-#endif
-#ifdef GBODE_REF
-  l.qold = __ldcg(e); e += c;
 #endif
 #pragma unroll
   for (int j = 0; j < F::NP; ++j) l.f.p[j] = (R)P.p[(long long)j * P.n + l.idx];
@@ -2259,7 +2253,7 @@ struct Feed {
     tick = 0;
     polls = 0;
     slot = 0;
-    if (!CROWDED || !P.park_ctl) return;
+    if (!CROWDED) return;
     unsigned sm, w;
     asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
     asm volatile("mov.u32 %0, %%warpid;" : "=r"(w));
@@ -2298,8 +2292,6 @@ struct Feed {
     if (!CROWDED) return __any_sync(FULL, active) || __any_sync(FULL, !exhausted);
     const unsigned act = __ballot_sync(FULL, active);
     if (!__any_sync(FULL, exhausted)) return true;
-    if (!P.park_ctl) return act != 0 || __any_sync(FULL, !exhausted);
-
     const int at_work = __popc(act), idle = 32 - at_work;
     if (at_work > 0 && (quiet || (++tick & 15) != 0)) return true;
     int* ctl = P.park_ctl;
