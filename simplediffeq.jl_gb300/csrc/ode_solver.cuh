@@ -2266,9 +2266,10 @@ struct Feed {
     }
   }
 
-  /* true: go on (some lane may be active); false: the warp's work is done */
+  /* what the warp does next: it ends, asks again, or makes an attempt (some lane is active) */
+  enum Turn { DONE, AGAIN, ATTEMPT };
   template <class M, class PR, int D, class F, int NK, class KS>
-  __device__ __forceinline__ bool next(const KParams& P, Lane<PR, D, F, NK, KS>& l, bool& active, Totals& tot) {
+  __device__ __forceinline__ Turn next(const KParams& P, Lane<PR, D, F, NK, KS>& l, bool& active, Totals& tot) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const bool want = !active && !exhausted;
@@ -2289,11 +2290,11 @@ struct Feed {
         }
       }
     }
-    if (!CROWDED) return __any_sync(FULL, active) || __any_sync(FULL, !exhausted);
     const unsigned act = __ballot_sync(FULL, active);
-    if (!__any_sync(FULL, exhausted)) return true;
+    if (!CROWDED) return act ? ATTEMPT : __any_sync(FULL, !exhausted) ? AGAIN : DONE;
+    if (!__any_sync(FULL, exhausted)) return act ? ATTEMPT : AGAIN;
     const int at_work = __popc(act), idle = 32 - at_work;
-    if (at_work > 0 && (quiet || (++tick & 15) != 0)) return true;
+    if (at_work > 0 && (quiet || (++tick & 15) != 0)) return ATTEMPT;
     int* ctl = P.park_ctl;
     int v = 0;
     if (lane < 5) v = __ldcg(lane < 4 ? ctl + lane : slot);
@@ -2324,7 +2325,7 @@ struct Feed {
           active = true;
         }
         counted -= take;
-        return true;
+        return __any_sync(FULL, active) ? ATTEMPT : AGAIN;
       }
     } else if (at_work > 0 && free_lanes >= 32 && warps > P.park_min && (long long)here * P.park_slots >= warps) {
       int room = 0, base = 0;
@@ -2349,7 +2350,7 @@ struct Feed {
     }
     if (at_work > 0) {
       quiet = warps <= P.park_min && tail == head;
-      return true;
+      return ATTEMPT;
     }
     /* no work: end, unless parked trajectories count on this warp's lanes */
     int stay = 0;
@@ -2364,14 +2365,14 @@ struct Feed {
     if (stay) {
       ++polls;
       __nanosleep(1000);
-      return true;
+      return AGAIN;
     }
     counted = 0;
     return leave(P, lane);
   }
 
-  /* the warp ends; true if it was the last one and trajectories are still parked */
-  __device__ __forceinline__ bool leave(const KParams& P, int lane) {
+  /* the warp ends, unless it is the last one and trajectories are still parked */
+  __device__ __forceinline__ Turn leave(const KParams& P, int lane) {
     int again = 0;
     __threadfence();
     __syncwarp();
@@ -2386,7 +2387,7 @@ struct Feed {
         atomicAdd(slot, 1);
       }
     }
-    return __shfl_sync(0xffffffffu, again, 0) != 0;
+    return __shfl_sync(0xffffffffu, again, 0) ? AGAIN : DONE;
   }
 };
 
@@ -2405,8 +2406,9 @@ __device__ __forceinline__ void run_adaptive_persistent(const KParams& P, typena
   Feed feed;
   feed.init(P);
   for (;;) {
-    if (!feed.next<MM>(P, l, active, tot)) break;
-    if (!__any_sync(FULL, active)) continue;
+    const Feed::Turn turn = feed.next<MM>(P, l, active, tot);
+    if (turn == Feed::DONE) break;
+    if (turn == Feed::AGAIN) continue;
     ST::vote(l.k, active);
     if (active && adaptive_iter<MM, SAVES>(P, l, tot)) active = false;
   }
@@ -2510,8 +2512,9 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P, typename P
   };
 
   for (;;) {
-    if (!feed.next<MM>(P, l, active, tot)) break;
-    if (!__any_sync(FULL, active)) continue;
+    const Feed::Turn turn = feed.next<MM>(P, l, active, tot);
+    if (turn == Feed::DONE) break;
+    if (turn == Feed::AGAIN) continue;
     ST::vote(l.k, active);
     R nh[D], nc[D];
     Accepted<T> st;
@@ -2713,8 +2716,9 @@ __device__ __forceinline__ void run_adaptive_staged2(const KParams& P, typename 
   Feed feed;
   feed.init(P);
   for (;;) {
-    if (!feed.next<MM>(P, l, active, tot)) break;
-    if (!__any_sync(FULL, active)) continue;
+    const Feed::Turn turn = feed.next<MM>(P, l, active, tot);
+    if (turn == Feed::DONE) break;
+    if (turn == Feed::AGAIN) continue;
     ST::vote(l.k, active);
     R nh[D], nc[D];
     Accepted<T> st;
