@@ -1509,7 +1509,7 @@ template <bool SHARED, class M, class PR, int D, class F> struct StageTypes {
   typedef typename PR::R KS[M::NK][D];
   enum { SLICE = 1 };
   __device__ static __forceinline__ void bind(KS&, typename PR::R*) {}
-  __device__ static __forceinline__ void vote(KS&, bool) {}
+  __device__ static __forceinline__ void vote(KS&, bool, bool) {}
 };
 template <class M, class PR, int D, class F> struct StageTypes<true, M, PR, D, F> {
   typedef MInt<M, PR, D, F> Method;
@@ -1521,9 +1521,10 @@ template <class M, class PR, int D, class F> struct StageTypes<true, M, PR, D, F
     k.off = false;
     k.rest = 0;
   }
-  /* by all lanes of a warp before an attempt, active ones or not */
-  __device__ static __forceinline__ void vote(KS& k, bool active) {
-    k.off = __any_sync(0xffffffffu, active && k.rest > 0);
+  /* by all lanes of a warp before an attempt, active ones or not; alone: the
+   * warp has its sub-partition's FP64 pipe to itself */
+  __device__ static __forceinline__ void vote(KS& k, bool active, bool alone) {
+    k.off = alone || __any_sync(0xffffffffu, active && k.rest > 0);
   }
 };
 
@@ -2121,7 +2122,7 @@ __device__ __forceinline__ void run_adaptive_plain(const KParams& P) {
     /* all lanes of a warp together, for the vote */
     bool active = i < P.n && !adaptive_start<MM>(P, i, l, tot);
     while (__any_sync(0xffffffffu, active)) {
-      ST::vote(l.k, active);
+      ST::vote(l.k, active, false);
       if (active) active = !adaptive_iter<MM, true>(P, l, tot);
     }
   } else if (i < P.n) {
@@ -2409,7 +2410,7 @@ __device__ __forceinline__ void run_adaptive_persistent(const KParams& P, typena
     const Feed::Turn turn = feed.next<MM>(P, l, active, tot);
     if (turn == Feed::DONE) break;
     if (turn == Feed::AGAIN) continue;
-    ST::vote(l.k, active);
+    ST::vote(l.k, active, feed.quiet);
     if (active && adaptive_iter<MM, SAVES>(P, l, tot)) active = false;
   }
   flush_totals(P, tot);
@@ -2515,7 +2516,7 @@ __device__ __forceinline__ void run_adaptive_staged(const KParams& P, typename P
     const Feed::Turn turn = feed.next<MM>(P, l, active, tot);
     if (turn == Feed::DONE) break;
     if (turn == Feed::AGAIN) continue;
-    ST::vote(l.k, active);
+    ST::vote(l.k, active, feed.quiet);
     R nh[D], nc[D];
     Accepted<T> st;
     int r = TRY_REJECTED, njobs = 0;
@@ -2719,7 +2720,7 @@ __device__ __forceinline__ void run_adaptive_staged2(const KParams& P, typename 
     const Feed::Turn turn = feed.next<MM>(P, l, active, tot);
     if (turn == Feed::DONE) break;
     if (turn == Feed::AGAIN) continue;
-    ST::vote(l.k, active);
+    ST::vote(l.k, active, feed.quiet);
     R nh[D], nc[D];
     Accepted<T> st;
     int r = TRY_REJECTED, njobs = 0;
