@@ -413,12 +413,14 @@ bool use_integer_pipe(const ode_handle* h, const ode_solve_args* a, int sched) {
  * trajectories, 100 save points: 161.7 ms unstaged, 116.4 ms staged in
  * one-warp blocks with 29 KB rings, 121.3 with 36 KB, 128.8 with 48 KB).
  * The integer-pipe kernels, whose warps also hold their stages in shared
- * memory, take two-warp blocks with the smallest ring. */
+ * memory, take two-warp blocks with the smallest ring, and one-warp blocks in
+ * the plain schedule, whose grid then fills the SMs most evenly. */
 void default_shape(const ode_handle* h, const ode_solve_args* a, int sched, int* block, int* stage) {
   *block = 128;
   *stage = 12288;
   const bool staged = !std::strcmp(entry_kind(a->alg, sched, a->nsave), "staged");
   if (use_integer_pipe(h, a, sched)) {
+    if (sched == ODE_SCHED_PLAIN) *block = 32;
     if (staged) *stage = small_ring_bytes(a);
     while (*block > 32 && *block / 32 * (stage_slice_bytes(a) + (staged ? *stage : 0)) > (staged ? 40960 : 49152))
       *block /= 2;
@@ -1143,7 +1145,9 @@ int solve_impl(ode_handle* h, const ode_solve_args* a, ode_solve_out* o, ode_sol
     block = 32 * D;  /* D warps per 32 trajectories */
     gridx = (unsigned)((n + 31) / 32);
   } else if (sched == ODE_SCHED_PLAIN) {
-    block = plain_block(n, h->nsm, block);
+    /* a block of the integer-pipe kernels takes the shared memory it was
+     * compiled with, however few threads it is launched with */
+    if (!use_integer_pipe(h, a, sched)) block = plain_block(n, h->nsm, block);
     gridx = (unsigned)((n + block - 1) / block);
   } else {
     int nb = 0;
