@@ -287,20 +287,35 @@ bool use_fixed_split(const ode_handle* h, const ode_solve_args* a) {
 }
 
 /* Adaptive Tsit5 under the persistent schedules, for ensembles small enough
- * that a warp for every component of 32 trajectories still has an SM
- * sub-partition to itself (run_adaptive_split; with more than four components
- * the sub-partitions share evenly): a lone warp's attempt is its FP64
- * instructions at one in 64 cycles, and D warps share them.  Time of the one-
- * thread-per-trajectory kernel over this one's, Lorenz without and with 100
- * save points: 1 trajectory 1.55 and 1.31, 32 1.55 and 1.28, 500 1.70 and 1.26,
- * 2,000 1.59 and 1.18, 4,800 (150 blocks for 152 SMs) 1.26 and 1.03; 6,400, some
- * SMs with two blocks, 1.17 and 0.86.  Linear, 20 save points, 2,000: dimension
- * 4 1.54, dimension 2 1.15. */
+ * that the warps of 32 trajectories' components share the SM sub-partitions
+ * evenly (run_adaptive_split; with up to four components each has one to
+ * itself): a lone warp's attempt is its FP64 instructions at one in 64 cycles,
+ * and D warps share them.  Time of the one-thread-per-trajectory kernel over
+ * this one's, at 1 / 32 / 500 trajectories, half the last size, the last:
+ *   linear  no save points                  20                            100
+ *   D = 2   1.24 1.26 1.38 1.31 1.27   1.10 1.09 1.15 1.10 1.06   0.78 1.12 1.11 1.06 1.05
+ *       3   1.61 1.63 1.74 1.66 1.33   1.47 1.41 1.45 1.42 1.23   1.11 1.62 1.65 1.59 1.51
+ *       5   1.58 1.57 1.70 1.50 1.26   1.48 1.47 1.55 1.39 1.12   1.22 1.62 1.64 1.48 1.14
+ *       6   1.56 1.56 1.63 1.43 1.22   1.48 1.50 1.50 1.20 1.00   1.17 1.67 1.60 1.25 0.91
+ *       8   1.76 1.76 1.86 1.62 1.32   1.69 1.66 1.61 1.27 0.97   1.43 1.66 1.53 1.03 0.78
+ * Lorenz 1.27 to 1.71 without, 1.03 to 1.53 with save points; Van der Pol 1.14
+ * to 1.22 and 0.94 to 1.12.
+ * With save points the last size is half as large for two components and for
+ * more than five (Van der Pol, 20: 1.02 at 4,864, 0.95 at 9,728).  Where the save
+ * points decide, the staged kernel, which spreads a step's over a warp's lanes,
+ * has them: with two components from 33 on, Van der Pol from 65 (linear, 60
+ * points, 1 to 4,864 trajectories: 0.85 to 0.97), and where a warp's lanes are
+ * idle from 101 (linear, D = 3, 1 to 8 trajectories, 200: 0.78 to 1.09). */
 bool use_adaptive_split(const ode_handle* h, const ode_solve_args* a, int sched) {
   const bool separable = a->rhs == ODE_RHS_LORENZ || a->rhs == ODE_RHS_VANDERPOL || a->rhs == ODE_RHS_LINEAR;
-  return a->alg == ODE_ALG_ATSIT5 && sched != ODE_SCHED_PLAIN && separable && a->output == ODE_OUTPUT_STATE &&
-         a->precision == ODE_FP64 && a->controller != ODE_CTRL_REF && a->dim >= 2 && a->dim <= 8 &&
-         (ensemble_size(h, a) + 31) / 32 <= (int64_t)(a->dim <= 4 ? h->nsm * (4 / a->dim) : h->nsm * 4 / a->dim);
+  if (a->alg != ODE_ALG_ATSIT5 || sched == ODE_SCHED_PLAIN || !separable || a->output != ODE_OUTPUT_STATE ||
+      a->precision != ODE_FP64 || a->controller == ODE_CTRL_REF || a->dim < 2 || a->dim > 8)
+    return false;
+  const int64_t n = ensemble_size(h, a);
+  if (a->dim == 2 ? a->nsave > (a->rhs == ODE_RHS_VANDERPOL ? 64 : 32) : n < 32 && a->nsave > 100) return false;
+  const int warps = a->nsave > 0 && (a->dim == 2 || a->dim > 5) ? 2 : 4; /* an SM's */
+  const int64_t most = a->dim <= 4 ? h->nsm * (warps / a->dim) : h->nsm * warps / a->dim;
+  return (n + 31) / 32 <= most;
 }
 
 /* entry_kind, with the component-split kernels where they apply */
