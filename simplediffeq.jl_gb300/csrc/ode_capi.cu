@@ -680,14 +680,23 @@ int plain_block(int64_t n, int nsm, int maxb) {
  * sub-partitions to hold the same number of warps: for a few more warps than
  * there are sub-partitions some hold two, which share the FP64 pipe and end
  * last, while the others wait; with one warp on each the lanes that finish
- * first take the remaining trajectories.  Up to 1.4 warps a sub-partition
- * (27,238 trajectories); above, two warps hide more latency than that costs.
- * Time with a warp per 32 trajectories over the time so, Lorenz final states,
- * Lotka-Volterra with saveat, linear of dimension 4 with saveat, AVern7 Van der
- * Pol with saveat, AVern9 three-body: 20,000 trajectories 1.41, 1.16, 1.19,
- * 1.10, 1.25; 25,000 (the first three) 1.26, 1.05, 1.16; 32,000 1.06, 0.95,
- * 1.05, 1.02, 1.13; 38,900 (the first three) 0.92, 0.84, 0.95.  Single
- * precision gains nothing from it.
+ * first take the remaining trajectories.  Up to 1.2 warps a sub-partition
+ * (23,347 trajectories) of a state of at most three components, or of phases,
+ * whose sines keep a lone warp's pipe busy.  Time with a warp per 32
+ * trajectories over the time so, at 19,500 / 23,000 / 25,000 / 27,200:
+ *                      no save points               20 save points
+ *   ATsit5 Lorenz      1.41 1.31 1.26 1.19     1.10 1.03 1.00 0.94
+ *     Van der Pol      1.31 1.25 1.24 1.20     1.04 1.20 1.18 1.14
+ *     Lotka-Volterra   1.29 1.09 1.06 1.06     1.25 1.07 1.01 1.02
+ *     linear, D = 2    1.04 1.01 0.94 0.91     1.07 1.01 0.92 0.92
+ *     Kuramoto-12      1.15 1.24 1.34 1.45     1.13 1.19 1.00 1.07
+ *     linear, D = 4    1.19 0.98 1.04 1.00     1.18 0.96 1.01 0.94
+ *     linear, D = 8    0.93 1.05 1.05 1.05     0.96 0.80 0.84 0.84
+ *   AVern7 Lorenz      1.58 1.40 1.34 1.26     1.12 1.01 1.04 0.98
+ *     linear, D = 4    1.19 1.05 1.10 1.02     0.95 0.89 0.95 0.94
+ *   AVern9 Van der Pol 1.58 1.55    - 1.46     1.12 1.10    - 1.14
+ *     linear, D = 8    0.87 1.14    - 1.10     0.90 0.92    - 0.85
+ * Single precision gains nothing from it.
  *
  * Verner 9 without saveat has registers for more warps than its lanes gain
  * from: with two warps a sub-partition in FP64 and three in single precision,
@@ -698,7 +707,9 @@ int64_t even_blocks(const ode_handle* h, const ode_solve_args* a, int block) {
   const int64_t warps = (a->n + 31) / 32, slots = (int64_t)h->nsm * 4;
   const int64_t most = a->alg == ODE_ALG_AVERN9 && a->nsave == 0 && block <= 128
                            ? slots * (a->precision == ODE_FP64 ? 2 : 3) / (block / 32) : INT64_MAX;
-  if (a->precision != ODE_FP64 || warps <= slots || warps * 10 > slots * 14 || block > 128) return most;
+  if (a->precision != ODE_FP64 || warps <= slots || warps * 10 > slots * 12 || block > 128 ||
+      (a->dim > 3 && a->rhs != ODE_RHS_KURAMOTO))
+    return most;
   return slots / (block / 32);
 }
 
