@@ -340,7 +340,8 @@ int kernel_kind_id(const char* k) {
  * trajectory index, the saveat index, and D (x2 with Kahan) state values,
  * DK x D stage values and, for the Verner methods, the parameters, of type R). */
 int stage_job_bytes(const ode_solve_args* a) {
-  const int nk = a->alg == ODE_ALG_AVERN9 ? 9 : 7;  /* the methods' DK */
+  const bool skips = a->precision == ODE_FP64;  /* the methods' DK */
+  const int nk = a->alg == ODE_ALG_AVERN9 ? (skips ? 9 : 16) : a->alg == ODE_ALG_AVERN7 && !skips ? 10 : 7;
   const int r = a->precision == ODE_FP64 ? 8 : 4, t = a->precision == ODE_FP32 ? 4 : 8;
   const bool dense_f = a->alg != ODE_ALG_ATSIT5;  /* Verner dense output evaluates f: parameters ride along */
   const int nrec = a->dim * (a->precision == ODE_FP32_KAHAN ? 2 : 1) + nk * a->dim + (dense_f ? a->nparams : 0);
@@ -355,7 +356,8 @@ int stage_job_bytes(const ode_solve_args* a) {
 int stage_record_bytes(const ode_solve_args* a) {
   const int nx = a->alg == ODE_ALG_AVERN9 ? 10 : a->alg == ODE_ALG_AVERN7 ? 6 : 0;
   if (!nx) return 0;
-  const int nk = a->alg == ODE_ALG_AVERN9 ? 9 : 7;
+  const bool skips = a->precision == ODE_FP64;
+  const int nk = a->alg == ODE_ALG_AVERN9 ? (skips ? 9 : 16) : skips ? 7 : 10;
   const int r = a->precision == ODE_FP64 ? 8 : 4, t = a->precision == ODE_FP32 ? 4 : 8;
   const int nrec = a->dim * (a->precision == ODE_FP32_KAHAN ? 2 : 1) + nk * a->dim + a->nparams + nx * a->dim;
   return 3 * t + 8 + 4 + nrec * r + 2 * 8;
