@@ -389,17 +389,23 @@ int small_ring_bytes(const ode_solve_args* a) { return (36 * stage_unit_bytes(a)
  * fewer warps, which the integer pipe's latency needs; time of the register
  * kernel over the crowded one's on Van der Pol, 0 / 20 / 200 save points:
  * 50,000 trajectories 1.32 / 1.06 / 0.95, 100,000 1.26 / 1.07 / 1.02, 200,003
- * 1.23 / 1.10 / 1.05.  Plain schedule, where a lane interpolates its save points
- * alone from stages in shared memory, 0 / 20 / 50 / 100 / 200: 60,000 0.95 with
- * none, 120,000 1.12 / 1.41 / 1.28 / 1.22 / 0.98, 400,000 1.13 / 1.38 / 1.26 /
- * 1.18 / 0.95; so five warps, and no more than 100 save points.  Verner 9 on the
- * three-body problem: 0.95 to 1.05. */
+ * 1.23 / 1.10 / 1.05.  Verner 9 on the three-body problem: 0.95 to 1.05.
+ *
+ * Verner 7, plain schedule, where a lane interpolates its save points alone
+ * from stages in shared memory: five warps (60,000 without save points 0.95),
+ * and no more than 20 points (200,000 trajectories, 0 / 20 / 50 / 100 points:
+ * linear of dimension 3 1.37 / 1.14 / 0.76 / 0.57, Van der Pol 1.36 / 1.31 / 1.21 /
+ * 0.97, Lorenz 1.55 / 1.60 / 1.34 / 1.19).
+ *
+ * Not the three-body problem with adaptive Tsit5: a few close encounters set
+ * its time, and their lone lanes gain nothing from rows on the integer pipe
+ * (39,000 trajectories 0.90, 131,072 0.95 without save points). */
 bool crowded(const ode_handle* h, const ode_solve_args* a, int sched) {
   if ((a->alg != ODE_ALG_ATSIT5 && a->alg != ODE_ALG_AVERN7) || a->precision != ODE_FP64 ||
       a->controller == ODE_CTRL_REF)
     return false;
   const bool v7 = a->alg == ODE_ALG_AVERN7, plain = sched == ODE_SCHED_PLAIN;
-  if (v7 && plain && a->nsave > 100) return false;
+  if ((v7 && plain && a->nsave > 20) || (!v7 && a->rhs == ODE_RHS_R3BP)) return false;
   return ensemble_size(h, a) > (int64_t)h->nsm * 4 * (v7 && (plain || a->nsave > 0) ? 160 : 64);
 }
 
