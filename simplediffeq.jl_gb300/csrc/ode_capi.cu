@@ -432,9 +432,14 @@ bool use_integer_pipe(const ode_handle* h, const ode_solve_args* a, int sched) {
 /* Launch shape of an untuned run-time compiled kernel: 128 threads and 12 KB
  * staging rings, unless those rings cannot hold a round of 32 (a staged kernel
  * with large records): then one-warp blocks with the smallest ring that can,
- * up to 48 KB (measured on AVern9, restricted three-body problem, 65,536
+ * up to 44 KB (measured on AVern9, restricted three-body problem, 65,536
  * trajectories, 100 save points: 161.7 ms unstaged, 116.4 ms staged in
- * one-warp blocks with 29 KB rings, 121.3 with 36 KB, 128.8 with 48 KB).
+ * one-warp blocks with 29 KB rings, 121.3 with 36 KB, 128.8 with 48 KB; AVern7
+ * on linear of dimension 8, 131,072 trajectories, 20 save points: 35.6 unstaged,
+ * 37.8 with 46 KB).  Step records that leave a 12 KB ring 38 or fewer take
+ * one-warp blocks too: small ensembles spread over more SMs and larger ones
+ * more evenly (AVern9 on Van der Pol, 20 save points, 32 records: 500
+ * trajectories 5%, 39,000 18% slower in 128 threads).
  * The integer-pipe kernels, whose warps also hold their stages in shared
  * memory, take two-warp blocks with the smallest ring, and one-warp blocks in
  * the plain schedule, whose grid then fills the SMs most evenly. */
@@ -451,9 +456,9 @@ void default_shape(const ode_handle* h, const ode_solve_args* a, int sched, int*
   }
   if (!staged) return;
   const int unit = stage_unit_bytes(a);
-  if (12288 / unit >= 32) return;
+  if (12288 / unit > (a->precision == ODE_FP64 && stage_record_bytes(a) ? 38 : 31)) return;
   const int fit = (32 * unit + 511) / 512 * 512;
-  if (fit > 49152) return;  /* no ring holds a round: the kernel runs unstaged */
+  if (fit > 45056) return;  /* no ring holds a round: the kernel runs unstaged */
   *block = 32;
   *stage = fit;
 }
@@ -710,11 +715,15 @@ int plain_block(int64_t n, int nsm, int maxb) {
  * from: with two warps a sub-partition in FP64 and three in single precision,
  * against three and five, fewer trajectories share the pipe with the longest
  * one.  Restricted three-body problem, 150,000 in FP64 61.0 against 65.3 ms,
- * 131,072 in FP32 with compensation 3.6 against 3.8 ms. */
+ * 131,072 in FP32 with compensation 3.6 against 3.8 ms.  Verner 7 with saveat
+ * the same below the crowded sizes: Lorenz, whose kernel has registers for
+ * three, 39,000 trajectories 11.1 against 13.7 ms, 65,536 17.4 against 18.7. */
 int64_t even_blocks(const ode_handle* h, const ode_solve_args* a, int block) {
   const int64_t warps = (a->n + 31) / 32, slots = (int64_t)h->nsm * 4;
-  const int64_t most = a->alg == ODE_ALG_AVERN9 && a->nsave == 0 && block <= 128
-                           ? slots * (a->precision == ODE_FP64 ? 2 : 3) / (block / 32) : INT64_MAX;
+  const bool two_warps = (a->alg == ODE_ALG_AVERN9 && (a->nsave == 0 || a->precision == ODE_FP64)) ||
+                         (a->alg == ODE_ALG_AVERN7 && a->nsave > 0 && a->dim > 2 &&
+                          a->precision == ODE_FP64 && !crowded(h, a, ODE_SCHED_PERSISTENT));
+  const int64_t most = two_warps && block <= 128 ? slots * (a->precision == ODE_FP64 ? 2 : 3) / (block / 32) : INT64_MAX;
   if (a->precision != ODE_FP64 || warps <= slots || warps * 10 > slots * 12 || block > 128 ||
       (a->dim > 3 && a->rhs != ODE_RHS_KURAMOTO))
     return most;
