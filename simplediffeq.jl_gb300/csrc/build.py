@@ -88,9 +88,9 @@ GROUPS = {
 # rings (36 jobs) in two-warp blocks give 16 warps per SM (1M learned Lorenz
 # solve: 104.8 ms with 8 warps per SM, 92.5 with 10, 84.6 with 12, 80.5 with 14,
 # 77.1 with 16).
-# The three-body kernels in FP64 take one-warp blocks: a small ensemble's warps
-# spread over more SMs (1,000 trajectories 13.8 -> 13.4 ms, 16,384 17.1 -> 16.6,
-# 150,000 the same).
+# The prebuilt three-body kernels in FP64 take one-warp blocks: a small ensemble's
+# warps spread over more SMs (1,000 trajectories 13.8 -> 13.4 ms, 16,384 17.1 ->
+# 16.6 on one set of inputs and the same on others, 150,000 the same).
 SHAPES = {"r3bp64": (32, 12288), "lorenz_staged": (64, 24576), "vdp_staged": (64, 24576), "kuramoto_staged": (32, 26112),
           "lorenz_plain_crowded": (32, 12288), "vdp_plain_crowded": (32, 12288),
           "lorenz_staged_crowded": (64, 8704), "kuramoto_staged_crowded": (32, 26112),

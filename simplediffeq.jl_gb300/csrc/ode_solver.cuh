@@ -1589,7 +1589,9 @@ __device__ __forceinline__ void store_point(const KParams& P, long long idx, lon
     if constexpr (CROWDED && D >= 8) {
       /* the right-hand side's copy of the sine and cosine, for the instruction
        * cache (131,072 Kuramoto-12 trajectories 85.9 to 80.8 ms; a lone warp's
-       * rounds are shorter with one inline: 8,192 take 42.4, not 44.8 ms) */
+       * rounds are shorter with one inline: 8,192 take 42.4, not 44.8 ms).
+       * Small states, whose code fits it anyway, keep theirs inline; measured at
+       * 12 components. */
       double sn[D], cs[D], w[D];
 #pragma unroll
       for (int d = 0; d < D; ++d) w[d] = v[d];
@@ -2236,8 +2238,12 @@ __device__ __forceinline__ int flag_seen(const int* flag) {
  * is).  A warp looks once in 16 attempts: a look takes an L2 round trip, and
  * the emptier the warps get meanwhile, the fewer move (each attempt 11.8 ms,
  * once in 4 11.4, in 8 10.9, in 32 10.6, in 64 10.9).  Others: 131,072
- * Kuramoto-12 87.1 to 83.2 ms, 200,003 Van der Pol 34.5 to 33.8, 65,536 single-
- * precision three-body 26.6 to 25.9, 100,003 Lorenz final states 11.5 to 9.7.
+ * Kuramoto-12 87.1 to 83.2 ms, 200,003 Van der Pol 34.5 to 33.8, 100,003 Lorenz
+ * final states 11.5 to 9.7.
+ *
+ * An entry is used once.  A warp parks once, with at most 32 entries of the
+ * launch's lanes, and ends; the last one to end may come back (leave), but then
+ * parks again only above park_min others.
  *
  * Nothing waits on another warp: entries are taken only once their flags are
  * there, a warp out of work gives lanes that others count on a bounded number
@@ -2878,7 +2884,8 @@ __device__ __forceinline__ void run_adaptive_staged_or_persistent(const KParams&
  * points, and Verner 9 leaves the dense output's code out of its loop: 168 to 96
  * registers in FP32 with compensation, 238 to 154 in FP64, and the restricted
  * three-body problem's long lone trajectories, which wait on instruction
- * fetch, 3 to 5% and 1% faster (16,384 in FP32, tolerance 1e-6: 2.43 to 2.33 ms).
+ * fetch, up to 4% faster (16,384 in FP32, tolerance 1e-6: 2.43 to 2.33 ms; other
+ * inputs within the runs' spread).
  * So do the crowded kernels: 1,000,000 Lorenz 68.8 to 60.4 ms, 65,536 7.0 to
  * 6.6, 400,000 Van der Pol with Verner 7 22.7 to 21.8.
  * For the smaller methods otherwise the registers that go free bring more resident warps
