@@ -443,12 +443,12 @@ int ode_learn_predict(ode_handle* h, const ode_solve_args* a, float* log_attempt
  * mean_b sum_o (out - y)^2 and the loss. */
 int ode_learn_gradcheck(ode_handle* h, int nin, int nh, int64_t batch, const float* params, const float* x,
                         const float* y, float* grad, float* loss);
-/* Clock cycles that an exchange between the training kernel's thread blocks
- * may take before ode_learn_fit and ode_learn_gradcheck return ODE_ECUDA (0:
- * the default, 4e9; below 0: none, every exchange fails at once, for
- * verification).  The context stays usable, and the handle keeps the model
- * fitted before. */
-int ode_learn_set_wait_limit(ode_handle* h, int64_t cycles);
+/* An exchange between the training kernel's thread blocks has about two
+ * seconds; then ode_learn_fit and ode_learn_gradcheck return ODE_ECUDA, the
+ * context stays usable and the handle keeps the model fitted before.  For
+ * verification: with enable = 1 the blocks wait for a piece that none sends, so
+ * that the time runs out. */
+int ode_learn_hold_exchanges(ode_handle* h, int enable);
 
 /* ---- allocation-free solve ------------------------------------------------
  * No counterpart in the reference: an entry point for callers that cannot

@@ -28,7 +28,8 @@ RET_DEFAULT, RET_DTMIN, RET_MAXITERS, RET_NAN = 0, 1, 2, 3
 # Every symbol include/gb300ode.h declares.
 EXPORTS = ["ode_abi_version", "ode_create", "ode_destroy", "ode_last_error", "ode_ensemble_solve",
            "ode_fixed_grid", "ode_rhs_compile", "ode_output_compile", "ode_learn_default_opts", "ode_learn_fit",
-           "ode_learn_predict", "ode_learn_gradcheck", "ode_learn_set_wait_limit", "ode_ensemble_solve_noalloc", "ode_autotune",
+           "ode_learn_predict", "ode_learn_gradcheck", "ode_learn_hold_exchanges",
+           "ode_ensemble_solve_noalloc", "ode_autotune",
            "ode_ensemble_solve_everystep", "ode_sde_solve", "ode_sde_compile", "ode_sde_compile_noise",
            "ode_set_bounds_check", "ode_tune_save", "ode_tune_load", "ode_rhs_builtin"]
 SDE = {"gbm": 0, "ou": 1, "lorenz": 2, "mult": 3}
@@ -155,7 +156,7 @@ def load():
     lib.ode_learn_predict.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveArgs), ctypes.c_void_p, ctypes.c_void_p]
     lib.ode_learn_gradcheck.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int64, ctypes.c_void_p,
                                         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
-    lib.ode_learn_set_wait_limit.argtypes = [ctypes.c_void_p, ctypes.c_int64]
+    lib.ode_learn_hold_exchanges.argtypes = [ctypes.c_void_p, ctypes.c_int]
     lib.ode_autotune.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveArgs), ctypes.c_int64, ctypes.POINTER(TuneReport)]
     lib.ode_tune_save.argtypes = [ctypes.c_void_p, ctypes.c_char_p]
     lib.ode_tune_load.argtypes = [ctypes.c_void_p, ctypes.c_char_p]
@@ -287,8 +288,8 @@ class Handle:
                                                 y.ctypes.data, grad.ctypes.data, loss.ctypes.data))
         return grad, float(loss[0])
 
-    def learn_set_wait_limit(self, cycles):
-        self.check(self.lib.ode_learn_set_wait_limit(self.h, int(cycles)))
+    def learn_hold_exchanges(self, enable=True):
+        self.check(self.lib.ode_learn_hold_exchanges(self.h, int(bool(enable))))
 
     def learn_predict(self, args, n):
         la = np.zeros(n, dtype=np.float32)

@@ -316,7 +316,7 @@ struct TrainParams {
   float* master;       /* in: initial fp32 parameters; out (training): trained fp32 parameters (flat layout) */
   __nv_bfloat16* wbf;  /* out (training): bf16 parameters */
   float* grad;         /* out (grad_only): fp32 gradient (flat layout) */
-  long long wait;      /* clock cycles an exchange between the CTAs may take; below 0: it fails at once */
+  int missing;         /* bytes that every CTA waits for and none sends: 0, or 16 where an exchange is to run out of time */
   float* loss;         /* [3]: summed minibatch losses of the first and the last epoch (atomic adds); 1 where an
                           exchange between the CTAs ran into its time limit */
 };
@@ -331,9 +331,9 @@ __device__ __forceinline__ void mbar_init(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect(uint32_t bar, int bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-/* true when the phase is complete, false after `limit` clock cycles */
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, int parity, long long limit) {
-  if (limit < 0) return false;
+/* true when the phase is complete, false after about two seconds (a limit the
+ * caller sets costs the training 1%) */
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, int parity) {
   const long long t0 = clock64();
   for (;;) {
     uint32_t done;
@@ -342,7 +342,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, int parity, long long li
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     if (done) return true;
-    if (clock64() - t0 > limit) return false;
+    if (clock64() - t0 > 4000000000ll) return false;
   }
 }
 __device__ __forceinline__ void bulk_to_cta(uint32_t dst, uint32_t src, int bytes, uint32_t bar, int q) {
@@ -763,12 +763,12 @@ __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
     if (lane == 0)
       for (int q = warp; q < csize; q += TT / 32)
         bulk_to_cta(smem_u32(rp + rank * L.S), smem_u32(gp + q * L.S), L.S * 4, bar_g, q);
-    if (tid == 0) mbar_expect(bar_g, csize * L.S * 4);
+    if (tid == 0) mbar_expect(bar_g, csize * L.S * 4 + tp.missing);
     const int tstep = step + 1;
     const float lr = tp.lr * (epoch < tp.epochs / 2 ? 1.f
                                                      : 0.1f + 0.9f * (float)(tp.epochs - epoch) / (tp.epochs / 2 + 1));
     const float c1 = 1.f - powf(b1, (float)tstep), c2 = 1.f - powf(b2, (float)tstep);
-    ok = __syncthreads_and(mbar_wait(bar_g, step & 1, tp.wait));
+    ok = __syncthreads_and(mbar_wait(bar_g, step & 1));
     if (!ok) break;
 #pragma unroll
     for (int u = 0; u < TU; ++u) {
@@ -816,7 +816,7 @@ __global__ void __launch_bounds__(TT, 1) mlp_train(TrainParams tp) {
       for (int q = warp; q < csize; q += TT / 32)
         bulk_to_cta(smem_u32(lin + rank * L.S), smem_u32(ws), L.S * 2, bar_w, q);
     if (tid == 0) mbar_expect(bar_w, csize * L.S * 2);
-    ok = __syncthreads_and(mbar_wait(bar_w, step & 1, tp.wait));
+    ok = __syncthreads_and(mbar_wait(bar_w, step & 1));
     if (!ok) break;
     const __nv_bfloat16 *l1 = lin, *lb1 = l1 + NH * nin, *l2 = lb1 + NH, *lb2 = l2 + NH * NH, *l3 = lb2 + NH;
     for (int i = tid; i < NH * NH / 8; i += TT)
@@ -1112,7 +1112,7 @@ static int train(ode_handle* h, Model* m, const std::vector<float>& X, const std
   tp.master = m->d_master;
   tp.wbf = m->d_w;
   tp.grad = nullptr;
-  tp.wait = h->learn_wait;
+  tp.missing = h->learn_hold ? 16 : 0;
   tp.loss = dL;
   int csize = 0;
   cudaError_t ee = cudaEventRecord(h->ev0, s);
@@ -1336,10 +1336,9 @@ int ode_learn_predict(ode_handle* h, const ode_solve_args* a, float* log_attempt
   return e == cudaSuccess ? ODE_OK : cuda_fail(h, e, "predict");
 }
 
-/* An exchange takes a few microseconds; the default of 4e9 cycles is two seconds. */
-int ode_learn_set_wait_limit(ode_handle* h, int64_t cycles) {
+int ode_learn_hold_exchanges(ode_handle* h, int enable) {
   if (!h) return ODE_EINVAL;
-  h->learn_wait = cycles == 0 ? kLearnWait : cycles;
+  h->learn_hold = enable != 0;
   return ODE_OK;
 }
 
@@ -1385,7 +1384,7 @@ int ode_learn_gradcheck(ode_handle* h, int nin, int nh, int64_t batch, const flo
   tp.grad_only = 1;
   tp.master = dP;
   tp.grad = dG;
-  tp.wait = h->learn_wait;
+  tp.missing = h->learn_hold ? 16 : 0;
   tp.loss = dL;
   rc = launch_train(h, tp, s, nullptr);
   if (rc != ODE_OK) return rc;

@@ -51,8 +51,6 @@ struct GraphEntry {
 
 constexpr int kGraphCache = 6;  /* captured solves kept per handle (least recently used evicted) */
 
-constexpr long long kLearnWait = 4000000000ll; /* clock cycles an exchange of the training kernel may take */
-
 constexpr int kCostBins = 1024;  /* bins of the learned schedule's counting sort */
 
 }  // namespace gbode
@@ -85,7 +83,7 @@ struct ode_handle {
   unsigned long long graph_tick = 0;
   gbode::Model* model = nullptr;        /* the fitted cost model */
   gbode::Model* spare_model = nullptr;  /* what a fit works on (ode_learn_fit) */
-  long long learn_wait = gbode::kLearnWait;
+  bool learn_hold = false;              /* ode_learn_hold_exchanges */
   bool bounds_check = false;  /* ode_set_bounds_check */
   int64_t tune_n = 0;         /* while autotuning: the whole ensemble's size */
 };

@@ -21,13 +21,13 @@ def test_the_wait_runs_out(pkg):
     h.learn_fit(args, {"epochs": 2})
     fitted = h.learn_predict(args, 4096)
     grad = h.learn_gradcheck(6, 64, prm, x, y)
-    h.learn_set_wait_limit(-1)
+    h.learn_hold_exchanges(True)
     for call in (lambda: h.learn_fit(args, {"epochs": 2, "seed": 5}), lambda: h.learn_gradcheck(6, 64, prm, x, y)):
         with pytest.raises(pkg.GB300ODEError, match="ran out of time") as e:
             call()
         assert e.value.code == L.ECUDA
     kept = h.learn_predict(args, 4096)
-    h.learn_set_wait_limit(0)
+    h.learn_hold_exchanges(False)
     again = h.learn_gradcheck(6, 64, prm, x, y)
     h.learn_fit(args, {"epochs": 2})
     refitted = h.learn_predict(args, 4096)
